@@ -21,6 +21,7 @@ Y in and out), "host" (host Y in and out) or "smatrix" (host Y in, S out).
 from __future__ import annotations
 
 import math
+from dataclasses import replace
 from functools import lru_cache
 
 import numpy as np
@@ -42,18 +43,18 @@ def listed():
         # a MOLSCAT scattering run: N 6-36, every 10th JTOT, both parities, host Y in and S out
         {"name": "rotor_ldmd_smatrix", "kind": "rotor", "prop": "LDMD", "via": "smatrix", "jmax": 80, "jstep": 10,
          "energies": 128, "nstep": 800},
-        # the same run with Johnson's propagator on device buffers
-        {"name": "rotor_ldj_device", "kind": "rotor", "prop": "LDJ", "via": "device", "jmax": 16, "jstep": 4,
+        # the same run with Johnson's propagator
+        {"name": "rotor_ldj_smatrix", "kind": "rotor", "prop": "LDJ", "via": "smatrix", "jmax": 16, "jstep": 4,
          "energies": 192, "nstep": 300},
-        # and with the symplectic propagator (MA5), host buffers
-        {"name": "rotor_ldmg5_host", "kind": "rotor", "prop": "LDMG5", "via": "host", "jmax": 12, "jstep": 3,
+        # and with the symplectic propagator (MA5)
+        {"name": "rotor_ldmg5_smatrix", "kind": "rotor", "prop": "LDMG5", "via": "smatrix", "jmax": 12, "jstep": 3,
          "energies": 160, "nstep": 100},
         # blocks of 41-64 channels, ragged
-        {"name": "dense_n45_60", "kind": "dense", "prop": "LDMD", "via": "device", "ns": "45,52,60", "energies": 320,
-         "nstep": 60},
+        {"name": "dense_n45_60", "kind": "dense", "prop": "LDMD", "via": "device", "ns": "45,52,60", "energies": 400,
+         "nstep": 40},
         # blocks of 65-200 channels in one plan, through to S matrices
         {"name": "dense_n72_199", "kind": "dense", "prop": "LDMD", "via": "smatrix", "ns": "72,90,128,199",
-         "energies": 48, "nstep": 60},
+         "energies": 48, "nstep": 40},
         # mid-size blocks with Johnson's propagator
         {"name": "dense_ldj_n50_120", "kind": "dense", "prop": "LDJ", "via": "device", "ns": "50,85,120",
          "energies": 96, "nstep": 40},
@@ -79,13 +80,13 @@ def draw(rng):
                 "block": rng.choice([1, 2]), "nstep": logint(400, 4000)}
     if kind == "rotor":
         prop = rng.choice(["LDMD", "LDJ", "LDMG4", "LDMG5"])
-        return {"kind": "rotor", "prop": prop, "via": rng.choice(["device", "host", "smatrix"]),
+        return {"kind": "rotor", "prop": prop, "via": "smatrix",
                 "jmax": rng.randint(10, 80), "jstep": rng.randint(7, 20), "energies": logint(16, 128),
                 "nstep": logint(100, 500) // (3 if prop.startswith("LDMG") else 1)}
     if kind == "dense":
         ns = sorted(rng.randint(41, 200) for _ in range(rng.randint(1, 3)))
         return {"kind": "dense", "prop": rng.choice(["LDMD", "LDMD", "LDJ"]), "via": rng.choice(["device", "host", "smatrix"]),
-                "ns": ",".join(str(n) for n in ns), "energies": logint(8, 64), "nstep": logint(20, 60)}
+                "ns": ",".join(str(n) for n in ns), "energies": logint(8, 64), "nstep": logint(16, 40)}
     if kind == "large":
         n = logint(201, 1000)
         return {"kind": "dense", "prop": rng.choice(["LDMD", "LDMD", "LDJ"]), "via": "device", "ns": str(n),
@@ -96,7 +97,7 @@ def draw(rng):
         return {"kind": "ldma", "jtot": rng.randint(0, 30), "block": rng.choice([1, 2]), "energies": logint(16, 200),
                 "nstep": logint(40, 150)}
     return {"kind": "serve", "prop": rng.choice(["LDMD", "LDJ"]), "nmin": 8, "nmax": rng.randint(30, 128),
-            "systems": rng.randint(3, 6), "requests": logint(16, 96), "nstep": logint(30, 60)}
+            "systems": rng.randint(3, 6), "requests": logint(16, 96), "nstep": logint(16, 40)}
 
 
 # ---------------------------------------------------------------------------
@@ -125,7 +126,8 @@ def _rotor_coupling(jtot, block):
 
 @lru_cache(maxsize=2)
 def _sweep(nout, nin):
-    return alkali.config4_sweep(nout=nout, nin=nin)
+    """The alkali-pair sweep 15 GHz below the lowest threshold (bound states)."""
+    return replace(alkali.config4_sweep(nout=nout, nin=nin), energy_mhz=-15000.0)
 
 
 def _dense_slice(n, nstep, rng):
