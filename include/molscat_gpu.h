@@ -393,14 +393,14 @@ int mgpu_release(mgpu_server *server, long long ticket);
 int mgpu_server_in_flight(mgpu_server *server, int *batches, int *queued, size_t *bytes);
 
 /* Kernel family for the sizes two families cover (N <= 64): 0 = FP64
- * tensor-core (DMMA) 8x8 fragments, one warp (N <= 40) or one CTA per
+ * tensor-core (DMMA) 8x8 fragments, one warp (N <= 64) or one CTA per
  * matrix (the default); 1 = 4x4 register tiles with the scalar sweep.
  * Affects plans created afterwards; returns the previous setting. */
 int mgpu_set_kernel_family(int family);
 
 /* Kernel family for plans and servers created afterwards, for propagator
  * iprop (0 = both) and n_lo <= N <= n_hi -- the autotuner's per-bucket choice
- * (molscat_b200/autotune.py): 0 = the default order (one warp for N <= 40,
+ * (molscat_b200/autotune.py): 0 = the default order (one warp for N <= 64,
  * one CTA up to 200, batched large-N above), 1 = 4x4 register tiles
  * (N <= 64), 2 = the batched large-N kernels (any N).  The latest call
  * covering N wins; a family without a bucket for N falls back to the default.

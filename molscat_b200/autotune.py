@@ -4,7 +4,7 @@ For every N range of the bucket table the tuner times each kernel family
 that can hold it on a representative batch (a dense synthetic system of the
 range's largest N, many energies) and keeps the fastest:
 
-    0  the default order: one warp per matrix (N <= 40), one CTA per matrix
+    0  the default order: one warp per matrix (N <= 64), one CTA per matrix
        (N <= 200), the batched large-N kernels above
     1  4x4 register tiles with the scalar sweep (N <= 64)
     2  the batched large-N kernels (matrices in global memory, 64 pivots a

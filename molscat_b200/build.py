@@ -25,6 +25,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC",
     "-shared",
     "-diag-suppress", "177",
+    "--split-compile=0",  # the kernels compile on all cores
 ]
 
 

@@ -1,11 +1,10 @@
-// LDMD / LDJ kernels for 40 < N <= 200: one CTA (4-16 warps) per matrix.
+// LDMD / LDJ / LDMG kernels for 64 < N <= 200: one CTA (8-16 warps) per matrix.
 // Included by propagator.cu after kernels_frag.cuh.
 //
 // The lower 8x8 tiles of the matrix live in shared memory in the DMMA
-// accumulator layout of warp_dmma.cuh ([t][lane][s], 512 bytes a tile), so
-// VL and the 2HQ(C) table use exactly the same layout as the one-warp
-// kernels.  The block sweep is the same four-pivots-per-round algorithm
-// (warp_dmma.cuh states it):
+// accumulator layout ([t][lane][s], 512 bytes a tile; channels in their own
+// order, lane l holds (8I + l/4, 8J + 2(l%4) + s)), VL and the 2HQ(C) table too.
+// The block sweep is the four-pivots-per-round algorithm of warp_dmma.cuh:
 //   1. thread i gathers row i of the panel A[i, P] from the lower triangle
 //      and forms its operand rows c(i) = Lam A[i, P] (B) and
 //      -c(i)/delta (X); rows of P carry -Lam^T and Lam^T/delta;   barrier
@@ -551,7 +550,8 @@ ldmd_prop_cta_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
         }
         // reference-potential solutions (mdprop.f:143-164)
         for (int i = tid; i < n; i += C::NTHR) {
-            const double wref = wf::w_diag_frag<NT>(S, i, 2 * k - 1, ered);
+            const size_t e = (size_t)tix(i >> 3, i >> 3) * 64 + ((i & 7) * 4 + ((i & 7) >> 1)) * 2 + (i & 1);
+            const double wref = w_elem(S, S.ptab + (size_t)(2 * k - 1) * S.nham, (int)e, i, i, 2 * k - 1, ered, true);
             double y14, y23;
             ref_solutions(wref, half, y14, y23);
             s_y14[i] = y14;
@@ -730,7 +730,7 @@ ldj_prop_cta_kernel(const SysDev *__restrict__ systems, const JobDev *__restrict
 }
 
 // ---------------------------------------------------------------------------
-// MGPROP step loop on one CTA per job (40 < N <= 200): the one-warp
+// MGPROP step loop on one CTA per job (64 < N <= 200): the one-warp
 // kernel's stages (kernels_frag.cuh, ldmg_prop_frag_kernel) with Y as tiles
 // in shared memory and the CTA sweep for the inversions.
 // ---------------------------------------------------------------------------

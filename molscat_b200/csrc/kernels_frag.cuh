@@ -1,10 +1,14 @@
-// LDMD / LDJ kernels on DMMA fragments: one warp per matrix (N <= 40).
+// LDMD / LDJ / LDMG kernels on DMMA fragments: one warp per matrix (N <= 64).
 // Included by propagator.cu after SysDev, JobDev, ref_solutions.
 //
 // Fragment layout (see warp_dmma.cuh): for every lower 8x8 tile t and lane l,
-// the two doubles of element (8I + (l>>2), 8J + 2(l&3) + s) are stored at
-// [t][l][s], so one warp reads or writes a tile as 512 contiguous bytes.
+// the two doubles of positions (l>>2, 2(l&3) + s) of the tile, channels
+// 8I + chan_of(l>>2) and 8J + chan_of(2(l&3) + s), are stored at [t][l][s], so
+// one warp reads or writes a tile as 512 contiguous bytes.
 // VL is stored [term][t][l][s]; the 2HQ(C) table [step][t][l][s].
+//
+// Padding channels (N .. 8 NT - 1) are uncoupled; every kernel gives them a
+// positive diagonal before an inversion, so the sweep needs no test for them.
 #pragma once
 #include "warp_dmma.cuh"
 
@@ -13,56 +17,76 @@ namespace wf {
 
 constexpr int kWPB = 4;  // warps (matrices) per CTA
 
-// per-warp shared memory (doubles): panel, y14, y14', y23, the 2HQ(C) tile
+// Doubles of shared memory per warp: the sweep's buffers, five channel vectors
+// (y14, y14', y23 by position; EINT, CENT by channel) and one tiled matrix
+// (LDMD: 2HQ(C_k); LDJ: the parked Z).
 template <int NT>
 struct WarpSmem {
     static constexpr int PAN = G<NT>::WSM;
     static constexpr int VEC = G<NT>::NPAD;
     static constexpr int QD = G<NT>::NTL * 64;
-    static constexpr int DOUBLES = PAN + 3 * VEC + QD;
+    static constexpr int DOUBLES = PAN + 5 * VEC + QD;
     static constexpr size_t BYTES = (size_t)DOUBLES * 8;
 };
 
-// The coupling sum sum_l VL_l P_l(R_ir) on this lane's fragment (SUMLAM,
-// sumlam.f:29-36,74-86): the part of W(R) that does not depend on the
-// energy or on EINT/CENT.
-template <int NT>
-__device__ __forceinline__ void w_sum_frag(const SysDev &S, int lane, int ir, double (&w)[G<NT>::NTL][2])
+// f(t, I, J, sum0, sum1) for every tile with the coupling sum
+// sum_l VL_l P_l(R_ir) (SUMLAM, sumlam.f:29-36,74-86) of this lane's two
+// elements: the part of W(R) that does not depend on the energy or on
+// EINT/CENT.  Up to CH tiles' sums are formed together, so that their loads
+// overlap, and only those are held in registers.
+template <int NT, class F>
+__device__ __forceinline__ void w_sum_each(const SysDev &S, int lane, int ir, F &&f)
 {
     constexpr int NTL = G<NT>::NTL;
+    constexpr int CH = NTL <= 15 ? NTL : 9;
     const double *P = S.ptab + (size_t)ir * S.nham;
+    const double *V = S.vlt + lane * 2;
+    const int *IVT = S.ivt + lane * 2;
 #pragma unroll
-    for (int t = 0; t < NTL; ++t) w[t][0] = w[t][1] = 0.0;
-    for (int l = 0; l < S.nham; ++l) {
-        const double *v = S.vlt + (size_t)l * NTL * 64 + lane * 2;
-        if (S.ivlfl <= 0) {
-            const double pl = __ldg(P + l);
+    for (int t0 = 0; t0 < NTL; t0 += CH) {
+        double w[CH][2];
 #pragma unroll
-            for (int t = 0; t < NTL; ++t) {
-                const double2 x = __ldg(reinterpret_cast<const double2 *>(v + t * 64));
-                w[t][0] = fma(x.x, pl, w[t][0]);
-                w[t][1] = fma(x.y, pl, w[t][1]);
+        for (int u = 0; u < CH; ++u) w[u][0] = w[u][1] = 0.0;
+        for (int l = 0; l < S.nham; ++l) {
+            const double *v = V + ((size_t)l * NTL + t0) * 64;
+            if (S.ivlfl <= 0) {
+                const double pl = __ldg(P + l);
+#pragma unroll
+                for (int u = 0; u < CH; ++u)
+                    if (t0 + u < NTL) {
+                        const double2 x = __ldg(reinterpret_cast<const double2 *>(v + u * 64));
+                        w[u][0] = fma(x.x, pl, w[u][0]);
+                        w[u][1] = fma(x.y, pl, w[u][1]);
+                    }
+            } else {
+                const int *iv = IVT + ((size_t)l * NTL + t0) * 64;
+#pragma unroll
+                for (int u = 0; u < CH; ++u)
+                    if (t0 + u < NTL) {
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const double x = __ldg(v + u * 64 + s);
+                            if (x != 0.0) w[u][s] = fma(x, __ldg(P + __ldg(iv + u * 64 + s)), w[u][s]);
+                        }
+                    }
             }
-        } else {
-            const int *iv = S.ivt + (size_t)l * NTL * 64 + lane * 2;
-#pragma unroll
-            for (int t = 0; t < NTL; ++t)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const double x = __ldg(v + t * 64 + s);
-                    if (x != 0.0) w[t][s] = fma(x, __ldg(P + __ldg(iv + t * 64 + s)), w[t][s]);
-                }
         }
+#pragma unroll
+        for (int I = 0; I < NT; ++I)
+#pragma unroll
+            for (int J = 0; J <= I; ++J)
+                if (tix(I, J) >= t0 && tix(I, J) < t0 + CH) f(tix(I, J), I, J, w[tix(I, J) - t0][0], w[tix(I, J) - t0][1]);
     }
 }
 
 // The diagonal terms of W(R_ir) (HAMMAT, hammat.f:85-113): CENT/R^2 (the
 // 1e16 clamp), EINT, the confinement term, then -ERED.  x is the coupling
 // sum of channel i's diagonal element.
-__device__ __forceinline__ double w_diag_terms(const SysDev &S, int i, double x, double rsq, double conf, double ered)
+__device__ __forceinline__ double w_diag_terms(const SysDev &S, const double *eint, const double *cent, int i, double x,
+                                               double rsq, double conf, double ered)
 {
-    if (S.nrsq == 0) x += rsq * S.cent[i];
-    if (S.nconst == 0) x += S.eint[i];
+    if (S.nrsq == 0) x += rsq * cent[i];
+    if (S.nconst == 0) x += eint[i];
     if (S.conlen > 0.0) x += conf;
     return x - ered;
 }
@@ -78,49 +102,42 @@ __device__ __forceinline__ void w_radial(const SysDev &S, int ir, double &rsq, d
     }
 }
 
-template <int NT>
-__device__ __forceinline__ void w_diag_frag_terms(const SysDev &S, int lane, int ir, double ered,
-                                                  double (&w)[G<NT>::NTL][2])
+// Add the diagonal terms to this lane's elements (w0, w1) of diagonal tile I.
+__device__ __forceinline__ void w_diag_add(const SysDev &S, const double *eint, const double *cent, int lane, int I,
+                                           double rsq, double conf, double ered, double &w0, double &w1)
+{
+    const int i = frow(I, lane);
+    if ((lane & 3) == (lane >> 3) && i < S.n) {
+        const bool s = (lane >> 2) & 1;
+        const double x = w_diag_terms(S, eint, cent, i, s ? w1 : w0, rsq, conf, ered);
+        if (s) w1 = x;
+        else w0 = x;
+    }
+}
+
+// f(t, I, J, w0, w1) for every tile with W(R_ir) (HAMMAT + SUMLAM, hammat.f:85-113)
+// of this lane's two elements.
+template <int NT, class F>
+__device__ __forceinline__ void w_each(const SysDev &S, const double *eint, const double *cent, int lane, int ir,
+                                       double ered, F &&f)
 {
     double rsq, conf;
     w_radial(S, ir, rsq, conf);
-    const int r = lane >> 2, q = lane & 3;
-#pragma unroll
-    for (int I = 0; I < NT; ++I)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const int i = 8 * I + r;
-            if (r == 2 * q + s && i < S.n) w[tix(I, I)][s] = w_diag_terms(S, i, w[tix(I, I)][s], rsq, conf, ered);
-        }
+    w_sum_each<NT>(S, lane, ir, [&](int t, int I, int J, double w0, double w1) {
+        if (I == J) w_diag_add(S, eint, cent, lane, I, rsq, conf, ered, w0, w1);
+        f(t, I, J, w0, w1);
+    });
 }
 
-// W(R) on this lane's fragment (HAMMAT + SUMLAM, hammat.f:85-113).
+// EINT and CENT into this warp's shared memory.
 template <int NT>
-__device__ __forceinline__ void w_frag(const SysDev &S, int lane, int ir, double ered, bool diag_terms,
-                                       double (&w)[G<NT>::NTL][2])
+__device__ __forceinline__ void stage_channels(const SysDev &S, int lane, double *eint, double *cent)
 {
-    w_sum_frag<NT>(S, lane, ir, w);
-    if (diag_terms) w_diag_frag_terms<NT>(S, lane, ir, ered, w);
-}
-
-// W(R_2m) for the step loop: the coupling sum from the system's table when
-// it has one (the preparation wrote it), else from VL; then the diagonal.
-template <int NT>
-__device__ __forceinline__ void w_step_frag(const SysDev &S, int lane, int m, double ered, double (&w)[G<NT>::NTL][2])
-{
-    constexpr int NTL = G<NT>::NTL;
-    if (S.wt != nullptr) {
-        const double *src = S.wt + (size_t)m * NTL * 64 + lane * 2;
-#pragma unroll
-        for (int t = 0; t < NTL; ++t) {
-            const double2 x = __ldg(reinterpret_cast<const double2 *>(src + t * 64));
-            w[t][0] = x.x;
-            w[t][1] = x.y;
-        }
-    } else {
-        w_sum_frag<NT>(S, lane, 2 * m, w);
+    for (int i = lane; i < G<NT>::NPAD; i += 32) {
+        eint[i] = __ldg(S.eint + i);
+        cent[i] = __ldg(S.cent + i);
     }
-    w_diag_frag_terms<NT>(S, lane, 2 * m, ered, w);
+    __syncwarp();
 }
 
 // The coupling sum of W(R_ir)_ii for channel i.
@@ -128,8 +145,8 @@ template <int NT>
 __device__ __forceinline__ double w_diag_sum_frag(const SysDev &S, int i, int ir)
 {
     constexpr int NTL = G<NT>::NTL;
-    const int I = i >> 3, r = i & 7;
-    const int lane = r * 4 + (r >> 1), s = r & 1;  // lane holding (r, r) of tile (I, I)
+    const int I = i >> 3, r = pos_of(i & 7);
+    const int lane = r * 4 + (r >> 1), s = r & 1;  // lane holding position (r, r) of tile (I, I)
     const size_t e = (size_t)tix(I, I) * 64 + lane * 2 + s;
     const double *P = S.ptab + (size_t)ir * S.nham;
     double x = 0.0;
@@ -141,25 +158,17 @@ __device__ __forceinline__ double w_diag_sum_frag(const SysDev &S, int i, int ir
     return x;
 }
 
-// W(R)_ii (the DIAG array of HAMMAT) for channel i.
+// W(R_2k-1)_ii (the DIAG array of HAMMAT) for the step loop, the coupling sum
+// from the system's table when it has one.
 template <int NT>
-__device__ __forceinline__ double w_diag_frag(const SysDev &S, int i, int ir, double ered)
-{
-    double rsq, conf;
-    w_radial(S, ir, rsq, conf);
-    return w_diag_terms(S, i, w_diag_sum_frag<NT>(S, i, ir), rsq, conf, ered);
-}
-
-// W(R_2k-1)_ii for the step loop, the coupling sum from the system's table
-// when it has one.
-template <int NT>
-__device__ __forceinline__ double w_mid_diag_frag(const SysDev &S, int i, int k, double ered)
+__device__ __forceinline__ double w_mid_diag_frag(const SysDev &S, const double *eint, const double *cent, int i, int k,
+                                                  double ered)
 {
     double rsq, conf;
     w_radial(S, 2 * k - 1, rsq, conf);
     const double x = S.wd != nullptr ? __ldg(S.wd + (size_t)(k - 1) * G<NT>::NPAD + i)
                                      : w_diag_sum_frag<NT>(S, i, 2 * k - 1);
-    return w_diag_terms(S, i, x, rsq, conf, ered);
+    return w_diag_terms(S, eint, cent, i, x, rsq, conf, ered);
 }
 
 template <int NT>
@@ -197,11 +206,17 @@ __device__ __forceinline__ void store_full_frag(double *__restrict__ y, int n, i
             }
 }
 
+// Resident CTAs (of kWPB warps) per SM the register budgets are set for.
+#ifndef MGPU_FMB
+#define MGPU_FMB 8, 6, 5, 4, 3, 2, 2, 2
+#endif
+constexpr int kFragBlocks[8] = {MGPU_FMB};
+constexpr int frag_min_blocks(int nt) { return kFragBlocks[nt - 1]; }
 // ---------------------------------------------------------------------------
 // MDPROP energy-independent half on fragments: grid (ceil(NSTEP/kWPB), systems).
 // ---------------------------------------------------------------------------
 template <int NT>
-__global__ void __launch_bounds__(32 * kWPB)
+__global__ void __launch_bounds__(32 * kWPB, frag_min_blocks(NT))
 ldmd_prep_frag_kernel(const SysDev *__restrict__ systems, const int *__restrict__ sys_list)
 {
     constexpr int NTL = G<NT>::NTL;
@@ -216,36 +231,23 @@ ldmd_prep_frag_kernel(const SysDev *__restrict__ systems, const int *__restrict_
     const double h = S.dr / 2.0;
     const double d1 = h * h / 3.0;
     const double d4 = -d1 / 16.0;
-    double a[NTL][2];
     if (S.wt != nullptr) {
         // the step loop's coupling sums: W at R_2k (and R_0 for the first
         // step) and the diagonal at R_2k-1, the same arithmetic as there
         for (int m = (k == 1 ? 0 : k); m <= k; ++m) {
-            w_sum_frag<NT>(S, lane, 2 * m, a);
             double *dst = S.wt + (size_t)m * NTL * 64 + lane * 2;
-#pragma unroll
-            for (int t = 0; t < NTL; ++t)
-                *reinterpret_cast<double2 *>(dst + t * 64) = make_double2(a[t][0], a[t][1]);
+            w_sum_each<NT>(S, lane, 2 * m, [&](int t, int, int, double w0, double w1) {
+                *reinterpret_cast<double2 *>(dst + t * 64) = make_double2(w0, w1);
+            });
         }
     }
-    w_sum_frag<NT>(S, lane, 2 * k - 1, a);
-    if (S.wd != nullptr) {
-        const int r = lane >> 2, q = lane & 3;
-#pragma unroll
-        for (int I = 0; I < NT; ++I)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
-                if (r == 2 * q + s) S.wd[(size_t)(k - 1) * G<NT>::NPAD + 8 * I + r] = a[tix(I, I)][s];
-    }
-#pragma unroll
-    for (int I = 0; I < NT; ++I)
-#pragma unroll
-        for (int J = 0; J <= I; ++J)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const int i = frow(I, lane), j = fcol(J, lane, s);
-                a[tix(I, J)][s] = (i == j) ? (i < S.n ? 0.125 : 0.0) : d4 * a[tix(I, J)][s];
-            }
+    double a[NTL][2];
+    w_sum_each<NT>(S, lane, 2 * k - 1, [&](int t, int I, int J, double w0, double w1) {
+        if (I == J && S.wd != nullptr && (lane & 3) == (lane >> 3))
+            S.wd[(size_t)(k - 1) * G<NT>::NPAD + frow(I, lane)] = ((lane >> 2) & 1) ? w1 : w0;
+        a[t][0] = (I == J && fdiag(lane, 0)) ? 0.125 : d4 * w0;
+        a[t][1] = (I == J && fdiag(lane, 1)) ? 0.125 : d4 * w1;
+    });
     int bad = SWEEP_OK;
     const int cnt = warp_sweep_invert<NT>(a, pans[warp], S.n, lane, bad);
     if (bad != SWEEP_OK) {
@@ -271,12 +273,6 @@ ldmd_prep_frag_kernel(const SysDev *__restrict__ systems, const int *__restrict_
         }
 }
 
-// Resident CTAs per SM the register budget is set for: NT = 5 (N 33-40) is
-// capped at 168 registers, three CTAs (12 warps) per SM hiding more of the
-// per-round latency than its few spills cost (+7 % at N = 36); the smaller NT
-// keep the occupancy their natural register counts give (an unconstrained
-// bound lets the compiler spend registers and lose a CTA per SM).
-constexpr int frag_min_blocks(int nt) { return nt <= 1 ? 5 : (nt <= 3 ? 4 : 3); }
 // ---------------------------------------------------------------------------
 // MDPROP step loop, one warp per job.
 // ---------------------------------------------------------------------------
@@ -300,7 +296,9 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
     double *s_y14 = pan + W::PAN;
     double *s_y14b = s_y14 + W::VEC;
     double *s_y23 = s_y14b + W::VEC;
-    double *qbuf = s_y23 + W::VEC;
+    double *s_eint = s_y23 + W::VEC;
+    double *s_cent = s_eint + W::VEC;
+    double *qbuf = s_cent + W::VEC;
     const int n = S.n;
     const int nstep = S.nstep;
     const double ered = job.ered;
@@ -315,7 +313,13 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
         }
         return;
     }
-    for (int i = lane; i < NPAD; i += 32) s_y14[i] = s_y14b[i] = s_y23[i] = 0.0;
+    // by position; a padding channel's diagonal is then 1 or 2 at every inversion
+    for (int i = lane; i < NPAD; i += 32) {
+        s_y14[i] = 0.5;
+        s_y14b[i] = 1.0;
+        s_y23[i] = 0.0;
+    }
+    stage_channels<NT>(S, lane, s_eint, s_cent);
     if (lane == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -330,20 +334,17 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
     double *yj = y + job.yoff;
 
     double a[NTL][2];
-    {
-        double w[NTL][2];
-        load_lower_frag<NT>(yj, n, lane, a);
-        w_step_frag<NT>(S, lane, 0, ered, w);
-#pragma unroll
-        for (int t = 0; t < NTL; ++t)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) a[t][s] = h * a[t][s] + d1 * w[t][s];  // mdprop.f:89-93
-    }
+    load_lower_frag<NT>(yj, n, lane, a);
+    w_each<NT>(S, s_eint, s_cent, lane, 0, ered, [&](int t, int, int, double w0, double w1) {
+        a[t][0] = h * a[t][0] + d1 * w0;  // mdprop.f:89-93
+        a[t][1] = h * a[t][1] + d1 * w1;
+    });
     const int r = lane >> 2, q = lane & 3;
     int nodes = 0, status = MGPU_OK, kfail = 0;
     int issued = 1, consumed = 0;
     const unsigned long long t0 = global_ns();
     const uint32_t wait_limit = g_step_wait_limit;
+    const bool tabled = S.wt != nullptr;
     for (int k = 1; k <= nstep; ++k) {
         if (stop_poll_step(k)) {  // host cancel / time limit, lane 0's reading for the warp
             int stop = lane == 0 ? stop_requested(S.ctl, t0) : MGPU_OK;
@@ -357,19 +358,21 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
         // reference-potential solutions in the sector (mdprop.f:143-164)
         __syncwarp();
         for (int i = lane; i < n; i += 32) {
-            const double wref = w_mid_diag_frag<NT>(S, i, k, ered);
+            const double wref = w_mid_diag_frag<NT>(S, s_eint, s_cent, i, k, ered);
             double y14, y23;
             ref_solutions(wref, half, y14, y23);
-            s_y14[i] = y14;
-            s_y14b[i] = y14 - d1 * wref;
-            s_y23[i] = y23;
+            const int p = (i & ~7) + pos_of(i & 7);
+            s_y14[p] = y14;
+            s_y14b[p] = y14 - d1 * wref;
+            s_y23[p] = y23;
         }
         __syncwarp();
 #pragma unroll
-        for (int I = 0; I < NT; ++I)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
-                if (r == 2 * q + s) a[tix(I, I)][s] += s_y14b[8 * I + r];
+        for (int I = 0; I < NT; ++I) {
+            const double d = s_y14b[8 * I + r];
+            if (fdiag(lane, 0)) a[tix(I, I)][0] += d;
+            if (fdiag(lane, 1)) a[tix(I, I)][1] += d;
+        }
         int bad = SWEEP_OK;
         nodes += warp_sweep_invert<NT>(a, pan, n, lane, bad);
         if (bad != SWEEP_OK) {
@@ -377,43 +380,42 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
             kfail = k;
             break;
         }
-        const bool landed = mbar_wait_bounded(bar, (k - 1) & 1, wait_limit);
+        // copy m of the run (2HQ(C_1), W(R_2), 2HQ(C_2), ..; without a table of
+        // coupling sums only the former) completes phase (m - 1) & 1
+        const bool landed = mbar_wait_bounded(bar, consumed & 1, wait_limit);
         if (__any_sync(0xffffffffu, !landed)) {
             status = MGPU_ERR_TIMEOUT;
             kfail = k;
             break;
         }
-        consumed = k;
-        double yr[NT], yc[NT][2];
-#pragma unroll
-        for (int I = 0; I < NT; ++I) {
-            yr[I] = s_y23[8 * I + r];
-            yc[I][0] = s_y23[8 * I + 2 * q];
-            yc[I][1] = s_y23[8 * I + 2 * q + 1];
-        }
+        ++consumed;
         {
             const double *qs = qbuf + lane * 2;
             // Y = 2HQ(C) + 2 Y14 - Y23 Y^-1 Y23   (a holds -Y^-1), mdprop.f:156,181-185
 #pragma unroll
-            for (int I = 0; I < NT; ++I)
+            for (int I = 0; I < NT; ++I) {
+                const double yr = s_y23[8 * I + r];
 #pragma unroll
                 for (int J = 0; J <= I; ++J) {
                     const double2 qq = *reinterpret_cast<const double2 *>(qs + tix(I, J) * 64);
-                    a[tix(I, J)][0] = qq.x + yr[I] * a[tix(I, J)][0] * yc[J][0];
-                    a[tix(I, J)][1] = qq.y + yr[I] * a[tix(I, J)][1] * yc[J][1];
+                    const double2 yc = *reinterpret_cast<const double2 *>(s_y23 + 8 * J + 2 * q);
+                    a[tix(I, J)][0] = qq.x + yr * a[tix(I, J)][0] * yc.x;
+                    a[tix(I, J)][1] = qq.y + yr * a[tix(I, J)][1] * yc.y;
                 }
-#pragma unroll
-            for (int I = 0; I < NT; ++I)
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-                    if (r == 2 * q + s) a[tix(I, I)][s] += 2.0 * s_y14[8 * I + r];
+                const double d = 2.0 * s_y14[8 * I + r];
+                if (fdiag(lane, 0)) a[tix(I, I)][0] += d;
+                if (fdiag(lane, 1)) a[tix(I, I)][1] += d;
+            }
         }
-        // every lane has read 2HQ(C_k): the async proxy may refill the buffer
+        // every lane has read 2HQ(C_k): the async proxy may refill the buffer,
+        // with the coupling sums of this step's W while the second inversion runs
         __syncwarp();
-        if (lane == 0 && k + 1 <= nstep) {
-            fence_async_shared();
-            bulk_load(qbuf, S.q + (size_t)k * NTL * 64, qbytes, bar);
-            issued = k + 1;
+        if (tabled || k + 1 <= nstep) {
+            if (lane == 0) {
+                fence_async_shared();
+                bulk_load(qbuf, tabled ? S.wt + (size_t)k * NTL * 64 : S.q + (size_t)k * NTL * 64, qbytes, bar);
+            }
+            ++issued;
         }
         nodes += warp_sweep_invert<NT>(a, pan, n, lane, bad);
         if (bad != SWEEP_OK) {
@@ -423,20 +425,50 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
         }
         {
             const double dd = (k == nstep) ? d1 : d2;
-            double w[NTL][2];
-            w_step_frag<NT>(S, lane, k, ered, w);
+            if (tabled) {
+                const bool there = mbar_wait_bounded(bar, consumed & 1, wait_limit);
+                if (__any_sync(0xffffffffu, !there)) {
+                    status = MGPU_ERR_TIMEOUT;
+                    kfail = k;
+                    break;
+                }
+                ++consumed;
+            }
+            auto finish = [&](int t, int I, int J, double w0, double w1) {
+                const double yr = s_y23[8 * I + r];
+                const double2 yc = *reinterpret_cast<const double2 *>(s_y23 + 8 * J + 2 * q);
+                a[t][0] = dd * w0 + yr * a[t][0] * yc.x;
+                a[t][1] = dd * w1 + yr * a[t][1] * yc.y;
+                if (I == J) {
+                    const double d = s_y14b[8 * I + r];
+                    if (fdiag(lane, 0)) a[t][0] += d;
+                    if (fdiag(lane, 1)) a[t][1] += d;
+                }
+            };
+            if (tabled) {
+                double rsq, conf;
+                w_radial(S, 2 * k, rsq, conf);
+                const double *ws = qbuf + lane * 2;
 #pragma unroll
-            for (int I = 0; I < NT; ++I)
+                for (int I = 0; I < NT; ++I)
 #pragma unroll
-                for (int J = 0; J <= I; ++J)
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-                        a[tix(I, J)][s] = dd * w[tix(I, J)][s] + yr[I] * a[tix(I, J)][s] * yc[J][s];
-#pragma unroll
-            for (int I = 0; I < NT; ++I)
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-                    if (r == 2 * q + s) a[tix(I, I)][s] += s_y14b[8 * I + r];
+                    for (int J = 0; J <= I; ++J) {
+                        const double2 x = *reinterpret_cast<const double2 *>(ws + tix(I, J) * 64);
+                        double w0 = x.x, w1 = x.y;
+                        if (I == J) w_diag_add(S, s_eint, s_cent, lane, I, rsq, conf, ered, w0, w1);
+                        finish(tix(I, J), I, J, w0, w1);
+                    }
+                __syncwarp();
+                if (k + 1 <= nstep) {
+                    if (lane == 0) {
+                        fence_async_shared();
+                        bulk_load(qbuf, S.q + (size_t)k * NTL * 64, qbytes, bar);
+                    }
+                    ++issued;
+                }
+            } else {
+                w_each<NT>(S, s_eint, s_cent, lane, 2 * k, ered, finish);
+            }
         }
     }
     if (status != MGPU_OK && lane == 0 && issued > consumed) {
@@ -457,19 +489,26 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
 // LDPROP step loop, one warp per job (ldprop.f:46-147).
 // ---------------------------------------------------------------------------
 template <int NT>
-__global__ void __launch_bounds__(32 * kWPB)
+__global__ void __launch_bounds__(32 * kWPB, frag_min_blocks(NT))
 ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restrict__ jobs, int njobs,
                      double *__restrict__ y, int *__restrict__ nodes_out, int *__restrict__ status_out,
                      int *__restrict__ kfail_out)
 {
     constexpr int NTL = G<NT>::NTL;
-    __shared__ __align__(16) double pans[kWPB][G<NT>::WSM];
+    using W = WarpSmem<NT>;
+    extern __shared__ __align__(16) double dsm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int jix = blockIdx.x * kWPB + warp;
     if (jix >= njobs) return;
     const JobDev job = jobs[jix];
     const SysDev &S = systems[job.sys];
-    double *pan = pans[warp];
+    double *pan = dsm + (size_t)warp * W::DOUBLES;
+    double *s_eint = pan + W::PAN;
+    double *s_cent = s_eint + W::VEC;
+    // Z waits here while U is inverted: one matrix in registers leaves room for
+    // the occupancy that hides the sweep's latency (two of them at N = 40 held
+    // the kernel to two CTAs an SM, and above 40 do not fit)
+    double *zs = pan + W::PAN + 5 * W::VEC + lane * 2;
     const int n = S.n;
     const double ered = job.ered;
     const double h = S.dr / 2.0;
@@ -477,20 +516,15 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
     const double d2 = 2.0 * d1;
     const double d4 = -d1 / 16.0;
     double *yj = y + job.yoff;
-    const int r = lane >> 2, q = lane & 3;
+    const bool dg0 = fdiag(lane, 0), dg1 = fdiag(lane, 1);  // padding channels included
+    stage_channels<NT>(S, lane, s_eint, s_cent);
 
-    double z[NTL][2], u[NTL][2];
-    load_lower_frag<NT>(yj, n, lane, z);
-    w_frag<NT>(S, lane, 0, ered, true, u);
-#pragma unroll
-    for (int I = 0; I < NT; ++I)
-#pragma unroll
-        for (int J = 0; J <= I; ++J)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                z[tix(I, J)][s] = h * z[tix(I, J)][s] + d1 * u[tix(I, J)][s] + (dg ? 1.0 : 0.0);  // ldprop.f:46-51
-            }
+    double a[NTL][2];
+    load_lower_frag<NT>(yj, n, lane, a);
+    w_each<NT>(S, s_eint, s_cent, lane, 0, ered, [&](int t, int I, int J, double w0, double w1) {
+        a[t][0] = h * a[t][0] + d1 * w0 + (I == J && dg0 ? 1.0 : 0.0);  // ldprop.f:46-51
+        a[t][1] = h * a[t][1] + d1 * w1 + (I == J && dg1 ? 1.0 : 0.0);
+    });
     int nodes = 0, status = MGPU_OK, kfail = 0;
     const unsigned long long t0 = global_ns();
     for (int k = 1; k <= S.nstep; ++k) {
@@ -503,20 +537,16 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
                 break;
             }
         }
-        w_frag<NT>(S, lane, 2 * k - 1, ered, true, u);
-#pragma unroll
-        for (int I = 0; I < NT; ++I)
-#pragma unroll
-            for (int J = 0; J <= I; ++J)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                    u[tix(I, J)][s] = d4 * u[tix(I, J)][s] + (dg ? 0.125 : 0.0);  // ldprop.f:67-72
-                }
-        int bad = SWEEP_OK;
-        const int ncu = warp_sweep_invert<NT>(u, pan, n, lane, bad);  // ldprop.f:78
         int bad2 = SWEEP_OK;
-        const int ncz = warp_sweep_invert<NT>(z, pan, n, lane, bad2);  // ldprop.f:83
+        const int ncz = warp_sweep_invert<NT>(a, pan, n, lane, bad2);  // ldprop.f:83
+#pragma unroll
+        for (int t = 0; t < NTL; ++t) *reinterpret_cast<double2 *>(zs + t * 64) = make_double2(a[t][0], a[t][1]);
+        w_each<NT>(S, s_eint, s_cent, lane, 2 * k - 1, ered, [&](int t, int I, int J, double w0, double w1) {
+            a[t][0] = d4 * w0 + (I == J && dg0 ? 0.125 : 0.0);  // ldprop.f:67-72
+            a[t][1] = d4 * w1 + (I == J && dg1 ? 0.125 : 0.0);
+        });
+        int bad = SWEEP_OK;
+        const int ncu = warp_sweep_invert<NT>(a, pan, n, lane, bad);  // ldprop.f:78
         if (bad != SWEEP_OK || bad2 != SWEEP_OK) {
             status = (bad == SWEEP_ZERO || bad2 == SWEEP_ZERO) ? MGPU_ERR_INVERSION : MGPU_ERR_NONFINITE;
             kfail = k;
@@ -526,14 +556,13 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
 #pragma unroll
         for (int I = 0; I < NT; ++I)
 #pragma unroll
-            for (int J = 0; J <= I; ++J)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                    // Z = U^-1 - Z^-1 - 6I with u = -U^-1, z = -Z^-1 (ldprop.f:92-97)
-                    z[tix(I, J)][s] = -u[tix(I, J)][s] + z[tix(I, J)][s] - (dg ? 6.0 : 0.0);
-                }
-        const int ncz2 = warp_sweep_invert<NT>(z, pan, n, lane, bad);  // ldprop.f:99
+            for (int J = 0; J <= I; ++J) {
+                // Z = U^-1 - Z^-1 - 6I with a = -U^-1, z = -Z^-1 (ldprop.f:92-97)
+                const double2 z = *reinterpret_cast<const double2 *>(zs + tix(I, J) * 64);
+                a[tix(I, J)][0] = -a[tix(I, J)][0] + z.x - (I == J && dg0 ? 6.0 : 0.0);
+                a[tix(I, J)][1] = -a[tix(I, J)][1] + z.y - (I == J && dg1 ? 6.0 : 0.0);
+            }
+        const int ncz2 = warp_sweep_invert<NT>(a, pan, n, lane, bad);  // ldprop.f:99
         if (bad != SWEEP_OK) {
             status = bad == SWEEP_ZERO ? MGPU_ERR_INVERSION : MGPU_ERR_NONFINITE;
             kfail = k;
@@ -541,17 +570,11 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
         }
         nodes += ncz2 - ncu;
         const double dd = (k == S.nstep) ? d1 : d2;
-        w_frag<NT>(S, lane, 2 * k, ered, true, u);
-#pragma unroll
-        for (int I = 0; I < NT; ++I)
-#pragma unroll
-            for (int J = 0; J <= I; ++J)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                    // Z = D2 W(B) + 2I - Z^-1 (ldprop.f:114-131)
-                    z[tix(I, J)][s] = dd * u[tix(I, J)][s] + (dg ? 2.0 : 0.0) + z[tix(I, J)][s];
-                }
+        w_each<NT>(S, s_eint, s_cent, lane, 2 * k, ered, [&](int t, int I, int J, double w0, double w1) {
+            // Z = D2 W(B) + 2I - Z^-1 (ldprop.f:114-131)
+            a[t][0] = dd * w0 + (I == J && dg0 ? 2.0 : 0.0) + a[t][0];
+            a[t][1] = dd * w1 + (I == J && dg1 ? 2.0 : 0.0) + a[t][1];
+        });
     }
     if (status == MGPU_OK) {
         // Y = Z/H - I/H (ldprop.f:140-147)
@@ -559,13 +582,11 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
 #pragma unroll
         for (int I = 0; I < NT; ++I)
 #pragma unroll
-            for (int J = 0; J <= I; ++J)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const bool dg = (I == J) && (r == 2 * q + s);
-                    z[tix(I, J)][s] = hi * z[tix(I, J)][s] - (dg ? hi : 0.0);
-                }
-        store_full_frag<NT>(yj, n, lane, 1.0, z);
+            for (int J = 0; J <= I; ++J) {
+                a[tix(I, J)][0] = hi * a[tix(I, J)][0] - (I == J && dg0 ? hi : 0.0);
+                a[tix(I, J)][1] = hi * a[tix(I, J)][1] - (I == J && dg1 ? hi : 0.0);
+            }
+        store_full_frag<NT>(yj, n, lane, 1.0, a);
     }
     if (lane == 0) {
         status_out[job.out] = status;
@@ -606,13 +627,14 @@ __constant__ MGCoef c_mg[2] = MGPU_MG_COEFS;
 #undef MGPU_MG_COEFS
 
 template <int NT>
-__global__ void __launch_bounds__(32 * kWPB)
+__global__ void __launch_bounds__(32 * kWPB, frag_min_blocks(NT))
 ldmg_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restrict__ jobs, int njobs, int method,
                       double *__restrict__ y, int *__restrict__ nodes_out, int *__restrict__ status_out,
                       int *__restrict__ kfail_out)
 {
     constexpr int NTL = G<NT>::NTL;
     __shared__ __align__(16) double pans[kWPB][G<NT>::WSM];
+    __shared__ double chan[kWPB][2 * G<NT>::NPAD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int jix = blockIdx.x * kWPB + warp;
     if (jix >= njobs) return;
@@ -624,9 +646,11 @@ ldmg_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
     const double ered = job.ered;
     const double h = S.dr;
     double *yj = y + job.yoff;
-    const int r = lane >> 2, q = lane & 3;
+    const bool dg0 = fdiag(lane, 0), dg1 = fdiag(lane, 1);  // padding channels included
+    double *s_eint = chan[warp], *s_cent = s_eint + G<NT>::NPAD;
+    stage_channels<NT>(S, lane, s_eint, s_cent);
 
-    double a[NTL][2], w[NTL][2];
+    double a[NTL][2];
     load_lower_frag<NT>(yj, n, lane, a);
     int nodes = 0, status = MGPU_OK, kfail = 0;
     const unsigned long long t0 = global_ns();
@@ -642,24 +666,21 @@ ldmg_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
         }
 #pragma unroll 1
         for (int k = 0; k < C.m; ++k) {
-            w_frag<NT>(S, lane, sec * C.stride + k, ered, true, w);
             const double bh = C.b[k] * h;
-#pragma unroll
-            for (int t = 0; t < NTL; ++t)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) a[t][s] = fma(bh, w[t][s], a[t][s]);  // X = Y + b_k h W
+            w_each<NT>(S, s_eint, s_cent, lane, sec * C.stride + k, ered, [&](int t, int, int, double w0, double w1) {
+                a[t][0] = fma(bh, w0, a[t][0]);  // X = Y + b_k h W
+                a[t][1] = fma(bh, w1, a[t][1]);
+            });
             const double ak = C.a[k];
             if (ak == 0.0) continue;  // Y = X
             const double ah = ak * h;
 #pragma unroll
             for (int I = 0; I < NT; ++I)
 #pragma unroll
-                for (int J = 0; J <= I; ++J)
-#pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                        a[tix(I, J)][s] = ah * a[tix(I, J)][s] + (dg ? 1.0 : 0.0);  // I + a_k h X
-                    }
+                for (int J = 0; J <= I; ++J) {
+                    a[tix(I, J)][0] = ah * a[tix(I, J)][0] + (I == J && dg0 ? 1.0 : 0.0);  // I + a_k h X
+                    a[tix(I, J)][1] = ah * a[tix(I, J)][1] + (I == J && dg1 ? 1.0 : 0.0);
+                }
             int bad = SWEEP_OK;
             const int cnt = warp_sweep_invert<NT>(a, pan, n, lane, bad);  // a = -(I + a_k h X)^-1
             if (bad != SWEEP_OK) {
@@ -672,12 +693,10 @@ ldmg_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
 #pragma unroll
             for (int I = 0; I < NT; ++I)
 #pragma unroll
-                for (int J = 0; J <= I; ++J)
-#pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        const bool dg = (I == J) && (r == 2 * q + s) && (8 * I + r < n);
-                        a[tix(I, J)][s] = (a[tix(I, J)][s] + (dg ? 1.0 : 0.0)) * d1;  // [I - inverse]/(a_k h)
-                    }
+                for (int J = 0; J <= I; ++J) {
+                    a[tix(I, J)][0] = (a[tix(I, J)][0] + (I == J && dg0 ? 1.0 : 0.0)) * d1;  // [I - inverse]/(a_k h)
+                    a[tix(I, J)][1] = (a[tix(I, J)][1] + (I == J && dg1 ? 1.0 : 0.0)) * d1;
+                }
         }
         if (status != MGPU_OK) break;
     }

@@ -36,7 +36,7 @@ constexpr int kT = 4;  // tile edge of every compiled bucket
 constexpr size_t kSmemBudget = 96 * 1024;  // dynamic shared memory per CTA we allow
 
 struct SysDev {
-    int n, nham, ivlfl, nconst, nrsq, nstep, ntiles, kind;  // kind: 0 = 4x4 register tiles, 1 = 8x8 DMMA fragments
+    int n, nham, ivlfl, nconst, nrsq, nstep, ntiles, kind;  // kind: the tile layout, tile_layout()
     double conlen, dr;
     const double *vlt;  // [nham][T*T][ntiles] tile layout, zero padding
     const int *ivt;     // same shape, 0-based P index (ivlfl > 0 only)
@@ -625,10 +625,12 @@ __global__ void __launch_bounds__(256) pivot_reciprocal_probe_kernel(const doubl
 // bucket dispatch
 // ---------------------------------------------------------------------------
 #define MGPU_BUCKETS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(16)
-#define MGPU_FRAG_BUCKETS(X) X(1) X(2) X(3) X(4) X(5)
+#ifndef MGPU_FRAG_BUCKETS
+#define MGPU_FRAG_BUCKETS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8)
+#endif
 // (NT, warps) of the one-CTA-per-matrix buckets, N = 8*NT up to 200
 #ifndef MGPU_CTA_BUCKETS
-#define MGPU_CTA_BUCKETS(X) X(6, 4) X(7, 4) X(8, 4) X(10, 8) X(12, 8) X(14, 8) X(16, 8) X(20, 16) X(25, 16)
+#define MGPU_CTA_BUCKETS(X) X(10, 8) X(12, 8) X(14, 8) X(16, 8) X(20, 16) X(25, 16)
 #endif
 
 // NT of the large-N buckets (matrices in global memory, 64 pivots a round):
@@ -646,7 +648,7 @@ struct Bucket {
     int warps;  // KIND_CTA8
 };
 
-// 8x8-fragment buckets first (one warp for N <= 40, one CTA up to 200), then
+// 8x8-fragment buckets first (one warp for N <= 64, one CTA up to 200), then
 // the 4x4 register tiles (N <= 64).
 static const Bucket kBuckets[] = {
 #define X(nt) {KIND_FRAG8, nt, 1},
@@ -665,6 +667,9 @@ static const Bucket kBuckets[] = {
 static const int kNumBuckets = sizeof(kBuckets) / sizeof(kBuckets[0]);
 
 static bool frag_layout(int b) { return kBuckets[b].kind != KIND_TILE4; }
+// 0 = 4x4 register tiles, 1 = 8x8 DMMA fragments, 2 = the same with the one-warp
+// kernels' channel order inside a tile (wf::chan_of)
+static int tile_layout(int b) { return !frag_layout(b) ? 0 : kBuckets[b].kind == KIND_FRAG8 ? 2 : 1; }
 static int bucket_edge(int b) { return frag_layout(b) ? 8 : kT; }
 static int bucket_npad(int b) { return bucket_edge(b) * kBuckets[b].nt; }
 static int ntiles_of(int b) { return kBuckets[b].nt * (kBuckets[b].nt + 1) / 2; }
@@ -823,7 +828,7 @@ static size_t prop_smem(int iprop, int b, int nham, int *vl_smem)
             MGPU_FRAG_BUCKETS(X)
 #undef X
         }
-        return iprop == MGPU_PROP_LDMD ? per * wf::kWPB : 0;
+        return is_ldmg(iprop) ? 0 : per * wf::kWPB;
     }
     const size_t tile_bytes = matrix_elems(b) * sizeof(double);
     const size_t base = iprop == MGPU_PROP_LDMD ? 2 * tile_bytes : 0;
@@ -872,8 +877,9 @@ static cudaError_t launch_prop(int iprop, int b, int njobs, size_t smem, int vl_
             wf::ldmg_prop_frag_kernel<t><<<blocks, 32 * wf::kWPB, 0, st>>>(                                   \
                 sys, jobs, njobs, iprop == MGPU_PROP_LDMG5 ? 1 : 0, y, nodes, status, kfail);                 \
         } else {                                                                                              \
-            wf::ldj_prop_frag_kernel<t><<<blocks, 32 * wf::kWPB, 0, st>>>(sys, jobs, njobs, y, nodes, status, \
-                                                                          kfail);                             \
+            if ((e = set_smem(wf::ldj_prop_frag_kernel<t>, smem))) return e;                                  \
+            wf::ldj_prop_frag_kernel<t><<<blocks, 32 * wf::kWPB, smem, st>>>(sys, jobs, njobs, y, nodes,      \
+                                                                             status, kfail);                  \
         }                                                                                                     \
         break;
             MGPU_FRAG_BUCKETS(X)
@@ -910,8 +916,13 @@ static void tile_element(int b, int t, int e, int *i, int *j)
     const int J = t - I * (I + 1) / 2;
     if (frag_layout(b)) {
         const int lane = e >> 1, s = e & 1;
-        *i = 8 * I + (lane >> 2);
-        *j = 8 * J + 2 * (lane & 3) + s;
+        int r = lane >> 2, c = 2 * (lane & 3) + s;
+        if (kBuckets[b].kind == KIND_FRAG8) {
+            r = wf::chan_of(r);
+            c = wf::chan_of(c);
+        }
+        *i = 8 * I + r;
+        *j = 8 * J + c;
     } else {
         *i = kT * I + e / kT;
         *j = kT * J + e % kT;
@@ -1233,7 +1244,7 @@ static int build_sysdev(const mgpu_coupling &c, const mgpu_grid &g, int iprop, i
     d.nrsq = c.nrsq;
     d.nstep = g.nstep;
     d.ntiles = nt;
-    d.kind = frag_layout(b) ? 1 : 0;
+    d.kind = tile_layout(b);
     d.conlen = c.conlen;
     d.dr = g.dr;
     // rows of the radial tables: MDPROP/LDPROP's half steps, MGPROP's stages
@@ -2507,7 +2518,7 @@ __global__ void noalloc_setup_kernel(SysDev proto, SysDev *sys_out, JobDev *jobs
         if (x < nvlt) {
             // x enumerates the destination array in its own layout
             int l, t, e;
-            if (proto.kind == 1) {  // [term][tile][lane][s]
+            if (proto.kind != 0) {  // [term][tile][lane][s]
                 e = (int)(x % TT);
                 t = (int)((x / TT) % nt);
                 l = (int)(x / ((size_t)TT * nt));
@@ -2520,10 +2531,16 @@ __global__ void noalloc_setup_kernel(SysDev proto, SysDev *sys_out, JobDev *jobs
             while ((I + 1) * (I + 2) / 2 <= t) ++I;
             const int J = t - I * (I + 1) / 2;
             int i, j;
-            if (proto.kind == 1) {
+            if (proto.kind != 0) {
                 const int lane = e >> 1, s2 = e & 1;
-                i = 8 * I + (lane >> 2);
-                j = 8 * J + 2 * (lane & 3) + s2;
+                i = lane >> 2;
+                j = 2 * (lane & 3) + s2;
+                if (proto.kind == 2) {
+                    i = wf::chan_of(i);
+                    j = wf::chan_of(j);
+                }
+                i += 8 * I;
+                j += 8 * J;
             } else {
                 i = I * edge + e / edge;
                 j = J * edge + e % edge;
@@ -2620,7 +2637,7 @@ extern "C" int mgpu_mdprop_noalloc(const mgpu_coupling *c, const mgpu_grid *g, i
     proto.nrsq = c->nrsq;
     proto.nstep = g->nstep;
     proto.ntiles = nt;
-    proto.kind = frag_layout(b) ? 1 : 0;
+    proto.kind = tile_layout(b);
     proto.conlen = c->conlen;
     proto.dr = g->dr;
     proto.vlt = reinterpret_cast<double *>(base + o_vlt);

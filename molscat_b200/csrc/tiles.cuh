@@ -69,6 +69,17 @@ __device__ __forceinline__ double pivot_reciprocal(double d)
     return fma(r, t, r) * sc;
 }
 
+// The same for a magnitude known to lie in [2^-1000, 2^1000): the scaling
+// factor would be one, so the result is the same bit for bit.
+__device__ __forceinline__ double pivot_reciprocal_plain(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    const double t = fma(e, e, e);
+    return fma(r, t, r);
+}
+
 // Publish column k (and 1/a_kk) into dst and zero this thread's entries of
 // row and column k.  Column k's lower part lives in tile column K, its upper
 // part (equal by symmetry) in tile row K.  Branch-free: predicated stores and

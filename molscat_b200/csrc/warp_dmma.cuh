@@ -2,9 +2,9 @@
 //
 // The matrix (padded to NPAD = 8*NT) is cut into 8x8 tiles; the lower
 // triangle of tiles, t = I*(I+1)/2 + J (I >= J), lives in registers in the
-// accumulator layout of mma.sync.m8n8k4.f64: lane l holds elements
-// (row 8I + (l>>2), col 8J + 2(l&3) + s), s = 0,1.  Diagonal tiles hold both
-// triangles.  Padding rows/columns are zero.
+// accumulator layout of mma.sync.m8n8k4.f64: lane l holds the elements at
+// positions (row l>>2, column 2(l&3) + s), s = 0,1, of a tile.  Diagonal tiles
+// hold both triangles.
 //
 // Inversion is the symmetric Gauss-Jordan sweep done four pivots at a time
 // (block sweep).  For the pivot block P = {p0..p0+3} with D = A_PP = L Delta L^T
@@ -16,13 +16,12 @@
 // sweep's own sum of rank-one terms, so the block sweep keeps its rounding
 // behaviour; forming D^{-1} first and updating with A_iP D^{-1} A_Pj instead
 // loses accuracy when a pivot is small next to its neighbours.  As in
-// tiles.cuh the owners zero row/column block P and the operands carry the
-// pivot block, so every lower tile gets the same update
+// tiles.cuh the entries of row/column block P are zeroed first and the operands
+// carry the pivot block, so every lower tile gets the same update
 //     A_IJ += X_I B_J          (one m8n8k4 DMMA per lower tile)
 // with X(i,k) = -c_k(i)/delta_k, B(j,k) = c_k(j) for rows outside P and
 // X(p0+a,k) = Lam[k][a]/delta_k, B(p0+b,k) = -Lam[k][b] for rows of P, which
-// writes A_iP D^{-1} into the columns of P and -D^{-1} into A_PP.  The panel
-// A_{:,P} goes through a small per-warp shared-memory buffer.  Every read of
+// writes A_iP D^{-1} into the columns of P and -D^{-1} into A_PP.  Every read of
 // a diagonal tile takes the lower triangle, so the stored matrix is symmetric
 // for the algorithm whatever rounding left in the upper triangle.
 //
@@ -44,8 +43,11 @@ template <int NT>
 struct G {
     static constexpr int NTL = NT * (NT + 1) / 2;  // lower tiles
     static constexpr int NPAD = 8 * NT;
-    static constexpr int PAN = NPAD * 4;           // panel doubles per warp
-    static constexpr int WSM = PAN + 16;           // panel + pivot-block buffer
+    // per-warp shared memory of the one-warp sweep (doubles): two pivot blocks,
+    // then a transposition buffer of NT - 1 tiles (rows 10 doubles apart: no
+    // bank conflict when a tile is read by columns)
+    static constexpr int TPITCH = 10;
+    static constexpr int WSM = 32 + (NT - 1) * 8 * TPITCH;
 };
 
 __host__ __device__ constexpr int tix(int I, int J) { return I * (I + 1) / 2 + J; }
@@ -58,6 +60,14 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
+}
+
+// D = X B + C with C in other registers than D.
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b, double c0, double c1)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%5};"
+                 : "=d"(d0), "=d"(d1)
+                 : "d"(a), "d"(b), "d"(c0), "d"(c1));
 }
 
 // Unpivoted LDL^T of the symmetric 4x4 pivot block D, read from the lower
@@ -103,22 +113,6 @@ __device__ __forceinline__ void ldl_block4(double d[4][4], int nreal, int &cnt, 
         for (int j = 0; j < 4; ++j) d[i][j] = (i == j) ? rd[i] : (i > j ? lam[i][j] : 0.0);
 }
 
-// Gather the 4x4 pivot block rows/cols 4H..4H+3 of diagonal tile (K, K)
-// into every lane with shuffles, lower triangle only: element (i, j), i >= j,
-// sits in lane (4H+i)*4 + 2H + (j>>1), slot j&1.  Ten shuffles.
-template <int NT, int K, int H>
-__device__ __forceinline__ void gather_block(const double (&a)[G<NT>::NTL][2], int lane, double (&f)[4][4])
-{
-    (void)lane;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            const int src = (4 * H + i) * 4 + 2 * H + (j >> 1);
-            f[i][j] = __shfl_sync(0xffffffffu, a[tix(K, K)][j & 1], src);
-        }
-}
-
 // This lane's share of the block operands (ldl_block4 layout in f): row q of
 // Lam below the diagonal (lq[m], m < q; zero for m >= q) and 1/delta_q.
 __device__ __forceinline__ void lane_operands(const double (&f)[4][4], int q, double (&lq)[3], double &rq)
@@ -129,138 +123,229 @@ __device__ __forceinline__ void lane_operands(const double (&f)[4][4], int q, do
     rq = (q == 1) ? f[1][1] : (q == 2) ? f[2][2] : (q == 3) ? f[3][3] : f[0][0];
 }
 
-// Lam[q][a] from this lane's row of Lam
-__device__ __forceinline__ double lam_qa(const double (&lq)[3], int q, int a)
+// ---- the one-warp sweep -----------------------------------------------------
+// Which channel of a tile's eight sits at position p of its rows and columns:
+// the even positions hold channels 3, 2, 1, 0 and the odd ones 7, 6, 5, 4.  A
+// four-pivot block is then one slot s of every lane, and a lane's element
+// A[i, P] (position 2q + s, pivot 3 - q of the block) is, as it stands in the
+// accumulators, an A operand of the DMMA: the panel needs no exchange between
+// lanes.  c = A[:, P] Lam^T is itself a DMMA (pivots in the order 3..0, so its
+// chain of FMAs runs 3, 2, 1, 0 as the scalar formula
+// fma(Lam0, A0, fma(Lam1, A1, fma(Lam2, A2, A3))) does, the leading terms being
+// exact), and its result is in the layout of the update's X and B operands.
+__host__ __device__ constexpr int chan_of(int p) { return 4 * (p & 1) + 3 - (p >> 1); }
+__host__ __device__ constexpr int pos_of(int c) { return 2 * (3 - (c & 3)) + (c >> 2); }
+
+// Pivots whose reciprocals need no scaling (and so are neither zero nor
+// non-finite): 2^-1000 <= |d| < 2^1000 for all four, from the exponent bits.
+__device__ __forceinline__ bool pivots_plain(double d0, double d1, double d2, double d3)
 {
-    const double x = (a == 0) ? lq[0] : (a == 1) ? lq[1] : (a == 2) ? lq[2] : 0.0;
-    return (a == q) ? 1.0 : x;
+    const unsigned a = (__double2hiint(d0) & 0x7fffffffu) - 0x01700000u, b = (__double2hiint(d1) & 0x7fffffffu) - 0x01700000u;
+    const unsigned c = (__double2hiint(d2) & 0x7fffffffu) - 0x01700000u, d = (__double2hiint(d3) & 0x7fffffffu) - 0x01700000u;
+    return max(max(a, b), max(c, d)) < 0x7d000000u;
 }
 
-// One block of four pivots, tile column K, half H (p0 = 8K + 4H).  f holds
-// the block's operands (ldl_block4) on entry and the next block's on exit
-// (computed right after the next block's diagonal tile is updated, so its
-// latency overlaps the rest of this block's DMMAs).
-template <int NT, int K, int H>
-__device__ __forceinline__ void sweep_round(double (&a)[G<NT>::NTL][2], double *pan, int n,
-                                            int lane, double (&f)[4][4], int &cnt, int &flags)
+// ldl_block4 with the exact scaling and the pivot flags, for a block that holds
+// an unusual pivot: blk[4i + j] (i >= j) in, the operands out in the same place.
+// Returns the negative pivots | flags << 8.
+__device__ __noinline__ int ldl_block4_any(double *blk)
+{
+    double d[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[i][j] = j <= i ? blk[4 * i + j] : 0.0;
+    int cnt = 0, flags = 0;
+    ldl_block4(d, 4, cnt, flags);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j) blk[4 * i + j] = d[i][j];
+    }
+    __syncwarp();
+    return cnt | (flags << 8);
+}
+
+// What the rounds need of a factored pivot block, per lane: lam = Lam[r>>1][3-q],
+// the B operand of c = A[:, P] Lam^T (its column 2k is pivot k), and
+// nrd = -1/delta_q.
+struct BlockOps {
+    double lam, nrd;
+};
+
+// Factor the pivot block of slot H of the diagonal tile (v: this lane's element
+// of that slot), ldl_block4's arithmetic in every lane.  The block reaches the
+// lanes through shared memory: one store and six loads against twenty shuffles
+// of four cycles each on the shared-memory pipe.  `live` = 0 (past the last
+// block of the matrix): nothing is counted.
+template <int H>
+__device__ __forceinline__ void factor_block(double v, double *blk, int lane, bool live, BlockOps &o, int &cnt,
+                                             int &flags)
 {
     const int r = lane >> 2, q = lane & 3;
-    constexpr int K2 = H ? K + 1 : K;  // next block
-    constexpr int H2 = H ? 0 : 1;
-    constexpr int p2 = 8 * K2 + 4 * H2;  // first pivot of the next block
-    // publish the panel A[i, P] (row i -> pan[4i .. 4i+3]) from the lower
-    // triangle: tiles below the diagonal in tile column K directly, tiles left
-    // of it in tile row K transposed; in diagonal tile K the rows of the other
-    // half come from whichever side of it lies in the lower triangle (rows of
-    // P themselves are not needed)
+    if ((r & 1) == H) blk[4 * (3 - (r >> 1)) + 3 - q] = v;
     __syncwarp();
-    if ((q >> 1) == H) {
-#pragma unroll
-        for (int I = (H ? K + 1 : K); I < NT; ++I) {
-            pan[(8 * I + r) * 4 + 2 * q - 4 * H] = a[tix(I, K)][0];
-            pan[(8 * I + r) * 4 + 2 * q - 4 * H + 1] = a[tix(I, K)][1];
-        }
+    const double2 b10 = *reinterpret_cast<const double2 *>(blk + 4);
+    const double2 b20 = *reinterpret_cast<const double2 *>(blk + 8);
+    const double2 b30 = *reinterpret_cast<const double2 *>(blk + 12);
+    const double2 b32 = *reinterpret_cast<const double2 *>(blk + 14);
+    double d00 = blk[0], d10 = b10.x, d11 = b10.y, d20 = b20.x, d21 = b20.y, d22 = blk[10];
+    double d30 = b30.x, d31 = b30.y, d32 = b32.x, d33 = b32.y;
+    double r0 = pivot_reciprocal_plain(d00);
+    double l10 = d10 * r0, l20 = d20 * r0, l30 = d30 * r0;
+    d11 = fma(-l10, d10, d11);
+    double r1 = pivot_reciprocal_plain(d11);
+    d21 = fma(-l20, d10, d21);
+    d31 = fma(-l30, d10, d31);
+    d22 = fma(-l20, d20, d22);
+    d32 = fma(-l30, d20, d32);
+    d33 = fma(-l30, d30, d33);
+    double l21 = d21 * r1, l31 = d31 * r1;
+    d22 = fma(-l21, d21, d22);
+    double r2 = pivot_reciprocal_plain(d22);
+    d32 = fma(-l31, d21, d32);
+    d33 = fma(-l31, d31, d33);
+    double l32 = d32 * r2;
+    d33 = fma(-l32, d32, d33);
+    double r3 = pivot_reciprocal_plain(d33);
+    // Lam = L^{-1} by forward substitution
+    double m10 = -l10, m21 = -l21, m32 = -l32;
+    double m20 = fma(-l21, m10, -l20);
+    double m31 = fma(-l32, m21, -l31);
+    double m30 = fma(-l32, m20, fma(-l31, m10, -l30));
+    int c = ((unsigned)__double2hiint(d00) >> 31) + ((unsigned)__double2hiint(d11) >> 31) +
+            ((unsigned)__double2hiint(d22) >> 31) + ((unsigned)__double2hiint(d33) >> 31);
+    if (!pivots_plain(d00, d11, d22, d33)) {  // the same in every lane
+        const int cf = ldl_block4_any(blk);
+        c = cf & 255;
+        flags |= live ? cf >> 8 : 0;
+        r0 = blk[0], m10 = blk[4], r1 = blk[5], m20 = blk[8], m21 = blk[9], r2 = blk[10];
+        m30 = blk[12], m31 = blk[13], m32 = blk[14], r3 = blk[15];
     }
-    if ((r >> 2) == H) {
-#pragma unroll
-        for (int J = 0; J < K; ++J) {
-            pan[(8 * J + 2 * q) * 4 + (r & 3)] = a[tix(K, J)][0];
-            pan[(8 * J + 2 * q + 1) * 4 + (r & 3)] = a[tix(K, J)][1];
-        }
-        if (H == 1 && q < 2) {
-            pan[(8 * K + 2 * q) * 4 + (r & 3)] = a[tix(K, K)][0];
-            pan[(8 * K + 2 * q + 1) * 4 + (r & 3)] = a[tix(K, K)][1];
-        }
-    }
-    __syncwarp();
-    double lq[3], rq;
-    lane_operands(f, q, lq, rq);
-    const double nrq = -rq;
-    // zero row/column block P
-#pragma unroll
-    for (int I = K; I < NT; ++I) {
-        a[tix(I, K)][0] = ((q >> 1) == H) ? 0.0 : a[tix(I, K)][0];
-        a[tix(I, K)][1] = ((q >> 1) == H) ? 0.0 : a[tix(I, K)][1];
-    }
-#pragma unroll
-    for (int J = 0; J <= K; ++J) {
-        a[tix(K, J)][0] = ((r >> 2) == H) ? 0.0 : a[tix(K, J)][0];
-        a[tix(K, J)][1] = ((r >> 2) == H) ? 0.0 : a[tix(K, J)][1];
-    }
-    // operands: X_I (A fragment: row r, col q), B_J (B fragment: row q, col r)
-    double X[NT], B[NT];
-#pragma unroll
-    for (int I = 0; I < NT; ++I) {
-        const double2 *row = reinterpret_cast<const double2 *>(pan + (8 * I + r) * 4);
-        const double2 x01 = row[0];
-        const double x2 = row[1].x;
-        const double vq = pan[(8 * I + r) * 4 + q];
-        const double c = fma(lq[0], x01.x, fma(lq[1], x01.y, fma(lq[2], x2, vq)));
-        X[I] = c * nrq;
-        B[I] = c;
-    }
-    if ((r >> 2) == H) {
-        // rows of P: X = Lam[q][a] / delta_q , B = -Lam[q][a]  (a = r & 3)
-        const double la = lam_qa(lq, q, r & 3);
-        X[K] = la * rq;
-        B[K] = -la;
-    }
-    // The next block's diagonal tile first; its operands are formed while the
-    // other DMMAs run.  Then the rest of the next panel's tile column and row,
-    // so the next round can publish early; the remaining tiles last.
-    if (K2 < NT) {
-        constexpr int KG = K2 < NT ? K2 : 0;
-        dmma(a[tix(KG, KG)][0], a[tix(KG, KG)][1], X[KG], B[KG]);
-        gather_block<NT, KG, H2>(a, lane, f);
-        ldl_block4(f, n - p2, cnt, flags);  // n - p2 <= 0: all padding, counts nothing
-#pragma unroll
-        for (int I = KG + 1; I < NT; ++I) dmma(a[tix(I, KG)][0], a[tix(I, KG)][1], X[I], B[KG]);
-#pragma unroll
-        for (int J = 0; J < KG; ++J) dmma(a[tix(KG, J)][0], a[tix(KG, J)][1], X[KG], B[J]);
-    }
-#pragma unroll
-    for (int I = 0; I < NT; ++I)
-#pragma unroll
-        for (int J = 0; J <= I; ++J)
-            if (I != K2 && J != K2) dmma(a[tix(I, J)][0], a[tix(I, J)][1], X[I], B[J]);
+    cnt += live ? c : 0;
+    const int j = r >> 1;  // row of Lam; this lane's column of it is 3 - q
+    const double c0 = j == 3 ? m30 : j == 2 ? m20 : m10;
+    const double c1 = j == 3 ? m31 : m21;
+    const double x = q == 3 ? c0 : q == 2 ? c1 : m32;
+    o.lam = j + q == 3 ? 1.0 : j + q > 3 ? x : 0.0;
+    o.nrd = -(q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3);
 }
 
-template <int NT, int R>
-struct Rounds {
-    static __device__ __forceinline__ void run(double (&a)[G<NT>::NTL][2], double *pan, int n, int lane,
-                                               double (&f)[4][4], int &cnt, int &flags)
-    {
-        constexpr int K = R / 2, H = R % 2;
-        if (8 * K + 4 * H < n) sweep_round<NT, K, H>(a, pan, n, lane, f, cnt, flags);
-        Rounds<NT, R + 1>::run(a, pan, n, lane, f, cnt, flags);
-    }
-};
-template <int NT>
-struct Rounds<NT, 2 * NT> {
-    static __device__ __forceinline__ void run(double (&)[G<NT>::NTL][2], double *, int, int, double (&)[4][4],
-                                               int &, int &)
-    {
-    }
-};
-
 // -A^{-1} in place; returns the negative-pivot count, `bad` as in tiles.cuh.
-// pan: G<NT>::PAN + 16 doubles of shared memory owned by this warp.
+// Padding rows and columns are uncoupled and have a positive diagonal.
+// ws: G<NT>::WSM doubles of shared memory owned by this warp.
+//
+// The loop runs over the tile columns with the pivot tile always the first:
+// after its two rounds every tile moves one place up and left (for nothing: the
+// update's result registers are simply other ones than its addend's), the tiles
+// of the first column become the last row, transposed through shared memory, and
+// after NT turns the matrix stands in its own order again.  Every register index
+// is fixed and the code is two rounds long, whatever NT: unrolled over the
+// rounds it filled the instruction caches (7843 instructions a propagation step
+// at NT = 5; this form issues about 3000), and with the pivot tile first there
+// is no row of tiles left of it, whose panel entries would need transposing.
+// The next block is factored as soon as its tile has its update, beside the
+// other DMMAs of the round.
 template <int NT>
-__device__ __forceinline__ int warp_sweep_invert(double (&a)[G<NT>::NTL][2], double *pan, int n, int lane, int &bad)
+__device__ __forceinline__ int warp_sweep_invert(double (&a)[G<NT>::NTL][2], double *ws, int n, int lane, int &bad)
 {
+    const int r = lane >> 2, q = lane & 3;
+    const bool odd = r & 1;
+    const double unit = q == (r >> 1) ? -1.0 : 0.0;  // rows of P: c = Lam (-I), exactly -Lam[k][a]
+    double *tb = ws + 32;
     int cnt = 0, flags = 0;
-    double f[4][4];
-    gather_block<NT, 0, 0>(a, lane, f);
-    ldl_block4(f, n, cnt, flags);
-    Rounds<NT, 0>::run(a, pan, n, lane, f, cnt, flags);
+    BlockOps f;
+    __syncwarp();
+    factor_block<0>(a[0][0], ws, lane, true, f, cnt, flags);
+#pragma unroll 1
+    for (int K = 0; K < NT; ++K) {
+        double B[NT], junk;
+        // first half: pivots in slot 0 of tile column 0 (X_I = B_I nrd, formed where it is used)
+        dmma(B[0], junk, odd ? a[0][0] : unit, f.lam, 0.0, 0.0);
+        dmma(a[0][0], a[0][1], B[0] * f.nrd, B[0], 0.0, odd ? a[0][1] : 0.0);
+#pragma unroll
+        for (int I = 1; I < NT; ++I) dmma(B[I], junk, a[tix(I, 0)][0], f.lam, 0.0, 0.0);
+        double nrd = f.nrd;
+        factor_block<1>(a[0][1], ws + 16, lane, 8 * K + 4 < n, f, cnt, flags);
+#pragma unroll
+        for (int I = 1; I < NT; ++I) {
+            const double X = B[I] * nrd;
+            dmma(a[tix(I, 0)][0], a[tix(I, 0)][1], X, B[0], 0.0, a[tix(I, 0)][1]);
+#pragma unroll
+            for (int J = 1; J <= I; ++J) dmma(a[tix(I, J)][0], a[tix(I, J)][1], X, B[J]);
+        }
+        // second half: slot 1; the rows of the first half take A[i, P] from the
+        // lower triangle, position (2q + 1, r)
+        const bool more = K + 1 < NT;
+        double e0, e1;  // the finished pivot tile
+        if (8 * K + 4 < n) {
+            const double up = __shfl_sync(0xffffffffu, a[0][0], (2 * q + 1) * 4 + (r >> 1));
+            dmma(B[0], junk, odd ? unit : up, f.lam, 0.0, 0.0);
+#pragma unroll
+            for (int I = 1; I < NT; ++I) dmma(B[I], junk, a[tix(I, 0)][1], f.lam, 0.0, 0.0);
+            nrd = f.nrd;
+            if constexpr (NT > 1) {
+                double d0, d1;  // the next pivot tile
+                dmma(d0, d1, B[1] * nrd, B[1], a[tix(1, 1)][0], a[tix(1, 1)][1]);
+                dmma(e0, e1, B[0] * nrd, B[0], odd ? 0.0 : a[0][0], 0.0);
+                a[0][0] = d0;
+                a[0][1] = d1;
+                factor_block<0>(a[0][0], ws, lane, more, f, cnt, flags);
+#pragma unroll
+                for (int I = 1; I < NT; ++I) {
+                    double t0, t1;
+                    const double X = B[I] * nrd;
+                    dmma(t0, t1, X, B[0], a[tix(I, 0)][0], 0.0);
+                    *reinterpret_cast<double2 *>(tb + ((I - 1) * 8 + r) * G<NT>::TPITCH + 2 * q) = make_double2(t0, t1);
+                    if (I > 1) {
+#pragma unroll
+                        for (int J = 1; J <= I; ++J)
+                            dmma(a[tix(I - 1, J - 1)][0], a[tix(I - 1, J - 1)][1], X, B[J], a[tix(I, J)][0], a[tix(I, J)][1]);
+                    }
+                }
+            } else {
+                dmma(e0, e1, B[0] * nrd, B[0], odd ? 0.0 : a[0][0], 0.0);
+            }
+        } else {  // the last tile column, its second half all padding: only the move
+            e0 = a[0][0];
+            e1 = a[0][1];
+            if constexpr (NT > 1) {
+#pragma unroll
+                for (int I = 1; I < NT; ++I)
+                    *reinterpret_cast<double2 *>(tb + ((I - 1) * 8 + r) * G<NT>::TPITCH + 2 * q) =
+                        make_double2(a[tix(I, 0)][0], a[tix(I, 0)][1]);
+#pragma unroll
+                for (int I = 1; I < NT; ++I)
+#pragma unroll
+                    for (int J = 1; J <= I; ++J) {
+                        a[tix(I - 1, J - 1)][0] = a[tix(I, J)][0];
+                        a[tix(I - 1, J - 1)][1] = a[tix(I, J)][1];
+                    }
+            }
+        }
+        if constexpr (NT > 1) {
+            __syncwarp();
+#pragma unroll
+            for (int J = 0; J + 1 < NT; ++J) {
+                a[tix(NT - 1, J)][0] = tb[(J * 8 + 2 * q) * G<NT>::TPITCH + r];
+                a[tix(NT - 1, J)][1] = tb[(J * 8 + 2 * q + 1) * G<NT>::TPITCH + r];
+            }
+        }
+        a[tix(NT - 1, NT - 1)][0] = e0;
+        a[tix(NT - 1, NT - 1)][1] = e1;
+    }
     bad = flags_to_status(flags);
     return cnt;
 }
 
 // ---- element bookkeeping ----------------------------------------------------
-// Row and column (global) of element s of tile (I, J) held by `lane`.
-__device__ __forceinline__ int frow(int I, int lane) { return 8 * I + (lane >> 2); }
-__device__ __forceinline__ int fcol(int J, int lane, int s) { return 8 * J + 2 * (lane & 3) + s; }
+// Channel of the row, and of column slot s, of tile (I, J) held by `lane`.
+__device__ __forceinline__ int frow(int I, int lane) { return 8 * I + chan_of(lane >> 2); }
+__device__ __forceinline__ int fcol(int J, int lane, int s) { return 8 * J + chan_of(2 * (lane & 3) + s); }
+// The lanes with (lane & 3) == lane >> 3 hold the diagonal of a diagonal tile, in slot (lane >> 2) & 1.
+__device__ __forceinline__ bool fdiag(int lane, int s) { return (lane >> 2) == 2 * (lane & 3) + s; }
 
 }  // namespace wf
 }  // namespace mgpu
