@@ -25,7 +25,6 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC",
     "-shared",
     "-diag-suppress", "177",
-    "--split-compile=0",  # the kernels compile on all cores
 ]
 
 

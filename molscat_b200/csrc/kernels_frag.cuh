@@ -336,8 +336,8 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
     double a[NTL][2];
     load_lower_frag<NT>(yj, n, lane, a);
     w_each<NT>(S, s_eint, s_cent, lane, 0, ered, [&](int t, int, int, double w0, double w1) {
-        a[t][0] = h * a[t][0] + d1 * w0;  // mdprop.f:89-93
-        a[t][1] = h * a[t][1] + d1 * w1;
+        a[t][0] = fma(h, a[t][0], d1 * w0);  // mdprop.f:89-93
+        a[t][1] = fma(h, a[t][1], d1 * w1);
     });
     const int r = lane >> 2, q = lane & 3;
     int nodes = 0, status = MGPU_OK, kfail = 0;
@@ -437,8 +437,8 @@ ldmd_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restri
             auto finish = [&](int t, int I, int J, double w0, double w1) {
                 const double yr = s_y23[8 * I + r];
                 const double2 yc = *reinterpret_cast<const double2 *>(s_y23 + 8 * J + 2 * q);
-                a[t][0] = dd * w0 + yr * a[t][0] * yc.x;
-                a[t][1] = dd * w1 + yr * a[t][1] * yc.y;
+                a[t][0] = fma(dd, w0, yr * a[t][0] * yc.x);
+                a[t][1] = fma(dd, w1, yr * a[t][1] * yc.y);
                 if (I == J) {
                     const double d = s_y14b[8 * I + r];
                     if (fdiag(lane, 0)) a[t][0] += d;
@@ -522,8 +522,8 @@ ldj_prop_frag_kernel(const SysDev *__restrict__ systems, const JobDev *__restric
     double a[NTL][2];
     load_lower_frag<NT>(yj, n, lane, a);
     w_each<NT>(S, s_eint, s_cent, lane, 0, ered, [&](int t, int I, int J, double w0, double w1) {
-        a[t][0] = h * a[t][0] + d1 * w0 + (I == J && dg0 ? 1.0 : 0.0);  // ldprop.f:46-51
-        a[t][1] = h * a[t][1] + d1 * w1 + (I == J && dg1 ? 1.0 : 0.0);
+        a[t][0] = fma(h, a[t][0], d1 * w0) + (I == J && dg0 ? 1.0 : 0.0);  // ldprop.f:46-51
+        a[t][1] = fma(h, a[t][1], d1 * w1) + (I == J && dg1 ? 1.0 : 0.0);
     });
     int nodes = 0, status = MGPU_OK, kfail = 0;
     const unsigned long long t0 = global_ns();

@@ -25,6 +25,7 @@
 #include <new>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "molscat_gpu.h"
@@ -628,10 +629,17 @@ __global__ void __launch_bounds__(256) pivot_reciprocal_probe_kernel(const doubl
 #ifndef MGPU_FRAG_BUCKETS
 #define MGPU_FRAG_BUCKETS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8)
 #endif
-// (NT, warps) of the one-CTA-per-matrix buckets, N = 8*NT up to 200
+// (NT, warps, warps in a launch of few jobs) of the one-CTA-per-matrix buckets,
+// N = 8*NT up to 200.  The results do not depend on the warps.  Measured, LDMD,
+// TFLOP/s with 1184 jobs: N = 72 6.3 on 4 warps (four CTAs an SM) against 4.5 on
+// 8; N = 106 6.5 on 8 against 4.3 on 12; N = 128 8.1 on 8 against 6.1 on 12;
+// N = 150 6.5 on 12 against 6.1 on 16.  With 48 jobs (one CTA an SM, a step's
+// latency): N = 72 46 us on 8 against 60 on 4; N = 128 106 on 12 against 125 on 8.
 #ifndef MGPU_CTA_BUCKETS
-#define MGPU_CTA_BUCKETS(X) X(10, 8) X(12, 8) X(14, 8) X(16, 8) X(20, 16) X(25, 16)
+#define MGPU_CTA_BUCKETS(X) X(10, 4, 8) X(12, 8, 8) X(14, 8, 8) X(16, 8, 12) X(20, 12, 12) X(25, 16, 16)
 #endif
+// Few jobs: the shape for them fills no more than one wave of the 148 SMs.
+static bool few_jobs(int njobs, int warps_few) { return njobs <= 148 * (warps_few <= 8 ? 2 : 1); }
 
 // NT of the large-N buckets (matrices in global memory, 64 pivots a round):
 // N up to 1024 in steps of 64
@@ -654,7 +662,7 @@ static const Bucket kBuckets[] = {
 #define X(nt) {KIND_FRAG8, nt, 1},
     MGPU_FRAG_BUCKETS(X)
 #undef X
-#define X(nt, w) {KIND_CTA8, nt, w},
+#define X(nt, w, wf) {KIND_CTA8, nt, w},
     MGPU_CTA_BUCKETS(X)
 #undef X
 #define X(nt) {KIND_BIG, nt, 0},
@@ -766,9 +774,9 @@ static cudaError_t launch_prep(int b, int max_nstep, int nsys, cudaStream_t st, 
         dim3 grid(max_nstep, nsys);
         cudaError_t e = cudaSuccess;
         switch (nt) {
-#define X(t, w)                                                                                   \
+#define X(t, w, wf)                                                                               \
     case t: {                                                                                     \
-        const size_t sm = cta::CSmem<t, w>::bytes(1);                                             \
+        const size_t sm = cta::CSmem<t, w>::bytes(false);                                             \
         if ((e = set_smem(cta::ldmd_prep_cta_kernel<t, w>, sm))) return e;                        \
         cta::ldmd_prep_cta_kernel<t, w><<<grid, 32 * w, sm, st>>>(sys, list);                    \
         break;                                                                                    \
@@ -814,7 +822,7 @@ static size_t prop_smem(int iprop, int b, int nham, int *vl_smem)
     if (kBuckets[b].kind == KIND_CTA8) {
         *vl_smem = 0;
         switch (kBuckets[b].nt) {
-#define X(t, w) case t: return cta::CSmem<t, w>::bytes(iprop == MGPU_PROP_LDJ ? 2 : 1);
+#define X(t, w, wf) case t: return cta::CSmem<t, w>::bytes(iprop == MGPU_PROP_LDJ);
             MGPU_CTA_BUCKETS(X)
 #undef X
         }
@@ -837,6 +845,27 @@ static size_t prop_smem(int iprop, int b, int nham, int *vl_smem)
     return base + (*vl_smem ? vlb : 0);
 }
 
+// The step kernels of a one-CTA bucket.
+template <int NT, int W>
+static cudaError_t launch_cta(int iprop, int njobs, cudaStream_t st, const SysDev *sys, const JobDev *jobs, double *y,
+                              int *nodes, int *status, int *kfail)
+{
+    const size_t smem = cta::CSmem<NT, W>::bytes(iprop == MGPU_PROP_LDJ);
+    cudaError_t e;
+    if (iprop == MGPU_PROP_LDMD) {
+        if ((e = set_smem(cta::ldmd_prop_cta_kernel<NT, W>, smem))) return e;
+        cta::ldmd_prop_cta_kernel<NT, W><<<njobs, 32 * W, smem, st>>>(sys, jobs, y, nodes, status, kfail);
+    } else if (is_ldmg(iprop)) {
+        if ((e = set_smem(cta::ldmg_prop_cta_kernel<NT, W>, smem))) return e;
+        cta::ldmg_prop_cta_kernel<NT, W><<<njobs, 32 * W, smem, st>>>(
+            sys, jobs, iprop == MGPU_PROP_LDMG5 ? 1 : 0, y, nodes, status, kfail);
+    } else {
+        if ((e = set_smem(cta::ldj_prop_cta_kernel<NT, W>, smem))) return e;
+        cta::ldj_prop_cta_kernel<NT, W><<<njobs, 32 * W, smem, st>>>(sys, jobs, y, nodes, status, kfail);
+    }
+    return cudaGetLastError();
+}
+
 static cudaError_t launch_prop(int iprop, int b, int njobs, size_t smem, int vl_smem, cudaStream_t st,
                                const SysDev *sys, const JobDev *jobs, double *y, int *nodes, int *status, int *kfail)
 {
@@ -844,25 +873,14 @@ static cudaError_t launch_prop(int iprop, int b, int njobs, size_t smem, int vl_
     const int nt = kBuckets[b].nt;
     if (kBuckets[b].kind == KIND_CTA8) {
         switch (nt) {
-#define X(t, w)                                                                                              \
-    case t:                                                                                                  \
-        if (iprop == MGPU_PROP_LDMD) {                                                                       \
-            if ((e = set_smem(cta::ldmd_prop_cta_kernel<t, w>, smem))) return e;                             \
-            cta::ldmd_prop_cta_kernel<t, w><<<njobs, 32 * w, smem, st>>>(sys, jobs, y, nodes, status, kfail); \
-        } else if (is_ldmg(iprop)) {                                                                         \
-            if ((e = set_smem(cta::ldmg_prop_cta_kernel<t, w>, smem))) return e;                             \
-            cta::ldmg_prop_cta_kernel<t, w><<<njobs, 32 * w, smem, st>>>(                                    \
-                sys, jobs, iprop == MGPU_PROP_LDMG5 ? 1 : 0, y, nodes, status, kfail);                       \
-        } else {                                                                                             \
-            if ((e = set_smem(cta::ldj_prop_cta_kernel<t, w>, smem))) return e;                              \
-            cta::ldj_prop_cta_kernel<t, w><<<njobs, 32 * w, smem, st>>>(sys, jobs, y, nodes, status, kfail);  \
-        }                                                                                                    \
-        break;
+#define X(t, w, wf)                                                                                  \
+    case t:                                                                                          \
+        return few_jobs(njobs, wf) ? launch_cta<t, wf>(iprop, njobs, st, sys, jobs, y, nodes, status, kfail) \
+                                   : launch_cta<t, w>(iprop, njobs, st, sys, jobs, y, nodes, status, kfail);
             MGPU_CTA_BUCKETS(X)
 #undef X
         default: return cudaErrorInvalidValue;
         }
-        return cudaGetLastError();
     }
     if (kBuckets[b].kind == KIND_FRAG8) {
         const int blocks = (njobs + wf::kWPB - 1) / wf::kWPB;

@@ -175,6 +175,51 @@ struct BlockOps {
     double lam, nrd;
 };
 
+// The operands of a factored 4x4 pivot block in registers: 1/delta_k and
+// Lam = L^{-1} below the diagonal.
+struct Block4 {
+    double r0, r1, r2, r3, m10, m20, m21, m30, m31, m32;
+};
+
+// ldl_block4's arithmetic for a block whose four pivots are plain
+// (pivots_plain); `neg` gets the negative ones.  Returns false when they are
+// not: the caller then takes ldl_block4_any.
+__device__ __forceinline__ bool ldl_block4_plain(double d00, double d10, double d11, double d20, double d21, double d22,
+                                                 double d30, double d31, double d32, double d33, Block4 &o, int &neg)
+{
+    o.r0 = pivot_reciprocal_plain(d00);
+    const double l10 = d10 * o.r0, l20 = d20 * o.r0, l30 = d30 * o.r0;
+    d11 = fma(-l10, d10, d11);
+    o.r1 = pivot_reciprocal_plain(d11);
+    d21 = fma(-l20, d10, d21);
+    d31 = fma(-l30, d10, d31);
+    d22 = fma(-l20, d20, d22);
+    d32 = fma(-l30, d20, d32);
+    d33 = fma(-l30, d30, d33);
+    const double l21 = d21 * o.r1, l31 = d31 * o.r1;
+    d22 = fma(-l21, d21, d22);
+    o.r2 = pivot_reciprocal_plain(d22);
+    d32 = fma(-l31, d21, d32);
+    d33 = fma(-l31, d31, d33);
+    const double l32 = d32 * o.r2;
+    d33 = fma(-l32, d32, d33);
+    o.r3 = pivot_reciprocal_plain(d33);
+    // Lam = L^{-1} by forward substitution
+    o.m10 = -l10, o.m21 = -l21, o.m32 = -l32;
+    o.m20 = fma(-l21, o.m10, -l20);
+    o.m31 = fma(-l32, o.m21, -l31);
+    o.m30 = fma(-l32, o.m20, fma(-l31, o.m10, -l30));
+    neg = ((unsigned)__double2hiint(d00) >> 31) + ((unsigned)__double2hiint(d11) >> 31) +
+          ((unsigned)__double2hiint(d22) >> 31) + ((unsigned)__double2hiint(d33) >> 31);
+    return pivots_plain(d00, d11, d22, d33);
+}
+
+__device__ __forceinline__ void block4_from(const double *blk, Block4 &o)
+{
+    o.r0 = blk[0], o.m10 = blk[4], o.r1 = blk[5], o.m20 = blk[8], o.m21 = blk[9], o.r2 = blk[10];
+    o.m30 = blk[12], o.m31 = blk[13], o.m32 = blk[14], o.r3 = blk[15];
+}
+
 // Factor the pivot block of slot H of the diagonal tile (v: this lane's element
 // of that slot), ldl_block4's arithmetic in every lane.  The block reaches the
 // lanes through shared memory: one store and six loads against twenty shuffles
@@ -191,46 +236,21 @@ __device__ __forceinline__ void factor_block(double v, double *blk, int lane, bo
     const double2 b20 = *reinterpret_cast<const double2 *>(blk + 8);
     const double2 b30 = *reinterpret_cast<const double2 *>(blk + 12);
     const double2 b32 = *reinterpret_cast<const double2 *>(blk + 14);
-    double d00 = blk[0], d10 = b10.x, d11 = b10.y, d20 = b20.x, d21 = b20.y, d22 = blk[10];
-    double d30 = b30.x, d31 = b30.y, d32 = b32.x, d33 = b32.y;
-    double r0 = pivot_reciprocal_plain(d00);
-    double l10 = d10 * r0, l20 = d20 * r0, l30 = d30 * r0;
-    d11 = fma(-l10, d10, d11);
-    double r1 = pivot_reciprocal_plain(d11);
-    d21 = fma(-l20, d10, d21);
-    d31 = fma(-l30, d10, d31);
-    d22 = fma(-l20, d20, d22);
-    d32 = fma(-l30, d20, d32);
-    d33 = fma(-l30, d30, d33);
-    double l21 = d21 * r1, l31 = d31 * r1;
-    d22 = fma(-l21, d21, d22);
-    double r2 = pivot_reciprocal_plain(d22);
-    d32 = fma(-l31, d21, d32);
-    d33 = fma(-l31, d31, d33);
-    double l32 = d32 * r2;
-    d33 = fma(-l32, d32, d33);
-    double r3 = pivot_reciprocal_plain(d33);
-    // Lam = L^{-1} by forward substitution
-    double m10 = -l10, m21 = -l21, m32 = -l32;
-    double m20 = fma(-l21, m10, -l20);
-    double m31 = fma(-l32, m21, -l31);
-    double m30 = fma(-l32, m20, fma(-l31, m10, -l30));
-    int c = ((unsigned)__double2hiint(d00) >> 31) + ((unsigned)__double2hiint(d11) >> 31) +
-            ((unsigned)__double2hiint(d22) >> 31) + ((unsigned)__double2hiint(d33) >> 31);
-    if (!pivots_plain(d00, d11, d22, d33)) {  // the same in every lane
-        const int cf = ldl_block4_any(blk);
+    Block4 b;
+    int c;
+    if (!ldl_block4_plain(blk[0], b10.x, b10.y, b20.x, b20.y, blk[10], b30.x, b30.y, b32.x, b32.y, b, c)) {
+        const int cf = ldl_block4_any(blk);  // the same in every lane
         c = cf & 255;
         flags |= live ? cf >> 8 : 0;
-        r0 = blk[0], m10 = blk[4], r1 = blk[5], m20 = blk[8], m21 = blk[9], r2 = blk[10];
-        m30 = blk[12], m31 = blk[13], m32 = blk[14], r3 = blk[15];
+        block4_from(blk, b);
     }
     cnt += live ? c : 0;
     const int j = r >> 1;  // row of Lam; this lane's column of it is 3 - q
-    const double c0 = j == 3 ? m30 : j == 2 ? m20 : m10;
-    const double c1 = j == 3 ? m31 : m21;
-    const double x = q == 3 ? c0 : q == 2 ? c1 : m32;
+    const double c0 = j == 3 ? b.m30 : j == 2 ? b.m20 : b.m10;
+    const double c1 = j == 3 ? b.m31 : b.m21;
+    const double x = q == 3 ? c0 : q == 2 ? c1 : b.m32;
     o.lam = j + q == 3 ? 1.0 : j + q > 3 ? x : 0.0;
-    o.nrd = -(q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3);
+    o.nrd = -(q == 0 ? b.r0 : q == 1 ? b.r1 : q == 2 ? b.r2 : b.r3);
 }
 
 // -A^{-1} in place; returns the negative-pivot count, `bad` as in tiles.cuh.
