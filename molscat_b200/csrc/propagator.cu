@@ -1077,6 +1077,16 @@ struct mgpu_plan {
         BigAux aux() const { return BigAux{side, evf, evj}; }
     };
     std::vector<BigStreams> bstreams;
+    // Streams of the small-N buckets after the first (which keeps the caller's):
+    // a bucket's step kernel runs as long as its longest propagation and, with
+    // few jobs, fills a part of the GPU, so one after the other the buckets'
+    // times added up (N 6-36 in three buckets: 31 ms; beside each other 16).
+    struct SmallStream {
+        cudaStream_t st = nullptr;
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<SmallStream> sstreams;
+    std::mutex run_mu;                     // a run's fork and join are queued by one thread at a time
     cudaStream_t own = nullptr;            // run_host's copies and launches
     cudaEvent_t ev_in = nullptr;
     // stop controls the step kernels poll: [0] cancel, [1] time budget (ns).
@@ -1103,6 +1113,11 @@ struct mgpu_plan {
         if (own) cudaStreamSynchronize(own);
         for (auto &q : bstreams)
             if (q.st) cudaStreamSynchronize(q.st);
+        for (auto &q : sstreams) {
+            if (q.st) cudaStreamSynchronize(q.st);
+            if (q.done) cudaEventDestroy(q.done);
+            if (q.st) cudaStreamDestroy(q.st);
+        }
         for (auto &g : big)
             if (g.step_graph) cudaGraphExecDestroy(g.step_graph);
         for (auto &q : bstreams) {
@@ -2014,6 +2029,19 @@ int mgpu_plan_create(mgpu_plan **out, int iprop, int nsys, const mgpu_coupling *
         }
         p->big.push_back(std::move(g));
     }
+    {
+        int nsmall = 0;
+        for (size_t slot = 0; slot < p->bucket_ids.size(); ++slot)
+            nsmall += kBuckets[p->bucket_ids[slot]].kind != KIND_BIG && p->job_count[slot] > 0;
+        if (nsmall > 1) p->sstreams.resize(nsmall - 1);
+        for (auto &q : p->sstreams)
+            if ((e = cudaStreamCreateWithFlags(&q.st, cudaStreamNonBlocking)) ||
+                (e = cudaEventCreateWithFlags(&q.done, cudaEventDisableTiming)) ||
+                (!p->ev_in && (e = cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming)))) {
+                delete p;
+                return set_err(MGPU_ERR_CUDA, "bucket streams", e);
+            }
+    }
     // inputs of Y -> S: the couplings' EINT and CENT, the grids' last radius
     p->s_ok = true;
     p->s_eint.resize(nsys);
@@ -2055,43 +2083,60 @@ int mgpu_plan_run_device_phases(mgpu_plan *p, double *y_dev, int *nodes_dev, int
         return set_err(MGPU_ERR_ARG, "null device buffer");
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
-    if (p->iprop == MGPU_PROP_LDMD && (phases & 1)) {
+    std::lock_guard<std::mutex> lk(p->run_mu);
+    const bool prep = p->iprop == MGPU_PROP_LDMD && (phases & 1);
+    if (prep) {
         // reset NSAVE / status / kfail of every system
         prep_reset_kernel<<<(p->nsys + 127) / 128, 128, 0, st>>>(p->d_prep, p->nsys);
         if ((e = cudaGetLastError())) return set_err(MGPU_ERR_CUDA, "launching prep_reset_kernel", e);
-        for (size_t b = 0; b < p->bucket_ids.size(); ++b) {
-            if (p->sys_count[b] == 0 || kBuckets[p->bucket_ids[b]].kind == KIND_BIG) continue;
-            for (int s0 = 0; s0 < p->sys_count[b]; s0 += 65535) {
-                if ((e = launch_prep(p->bucket_ids[b], p->max_nstep[b], std::min(65535, p->sys_count[b] - s0), st,
-                                     p->d_sys, p->d_syslists + p->sys_begin[b] + s0)))
-                    return set_err(MGPU_ERR_CUDA, "launching ldmd_prep_kernel", e);
-            }
-        }
     }
-    if (!p->big.empty()) {
-        // every large-N bucket on its own stream pair, ordered after the caller's stream
-        if ((e = cudaEventRecord(p->ev_in, st))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
-        for (size_t i = 0; i < p->big.size(); ++i) {
-            BigBucket &g = p->big[i];
-            const mgpu_plan::BigStreams &q = p->bstreams[i];
-            if ((e = cudaStreamWaitEvent(q.st, p->ev_in, 0))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
-            if (p->iprop == MGPU_PROP_LDMD && (phases & 1) &&
-                (e = run_big_prep(g, p->d_sys, p->sys_nstep, q.st, q.aux())))
-                return set_err(MGPU_ERR_CUDA, "large-N preparation", e);
-            if ((phases & 2) && (e = run_big_prop(g, p->iprop, p->d_sys, y_dev, nodes_dev, status_dev, kfail_dev,
-                                                  q.st, q.aux())))
-                return set_err(MGPU_ERR_CUDA, "large-N propagation", e);
-            if ((e = cudaEventRecord(q.done, q.st))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
-        }
+    // A caller capturing a graph gets the small-N buckets one after the other on its own stream.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!p->sstreams.empty() && (e = cudaStreamIsCapturing(st, &cap))) return set_err(MGPU_ERR_CUDA, "stream state", e);
+    const bool fork = !p->sstreams.empty() && cap == cudaStreamCaptureStatusNone;
+    if (fork || !p->big.empty()) {
+        // the buckets' own streams are ordered after the caller's
+        if ((e = cudaEventRecord(p->ev_in, st))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     }
-    // the small-N buckets on the caller's stream, beside the large-N streams
-    for (size_t b = 0; b < p->bucket_ids.size() && (phases & 2); ++b) {
-        if (p->job_count[b] == 0 || kBuckets[p->bucket_ids[b]].kind == KIND_BIG) continue;
-        if ((e = launch_prop(p->iprop, p->bucket_ids[b], p->job_count[b], p->smem[b], p->vl_smem[b], st, p->d_sys,
+    // every large-N bucket on its own stream pair
+    for (size_t i = 0; i < p->big.size(); ++i) {
+        BigBucket &g = p->big[i];
+        const mgpu_plan::BigStreams &q = p->bstreams[i];
+        if ((e = cudaStreamWaitEvent(q.st, p->ev_in, 0))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
+        if (prep && (e = run_big_prep(g, p->d_sys, p->sys_nstep, q.st, q.aux())))
+            return set_err(MGPU_ERR_CUDA, "large-N preparation", e);
+        if ((phases & 2) && (e = run_big_prop(g, p->iprop, p->d_sys, y_dev, nodes_dev, status_dev, kfail_dev,
+                                              q.st, q.aux())))
+            return set_err(MGPU_ERR_CUDA, "large-N propagation", e);
+        if ((e = cudaEventRecord(q.done, q.st))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
+    }
+    // the small-N buckets beside them: the first with jobs on the caller's
+    // stream, each of the others on one of its own
+    int nth = 0;
+    for (size_t b = 0; b < p->bucket_ids.size(); ++b) {
+        if (kBuckets[p->bucket_ids[b]].kind == KIND_BIG) continue;
+        const bool jobs = p->job_count[b] > 0;
+        const int side = jobs && fork ? nth - 1 : -1;
+        nth += jobs;
+        cudaStream_t bs = st;
+        if (side >= 0) {
+            bs = p->sstreams[side].st;
+            if ((e = cudaStreamWaitEvent(bs, p->ev_in, 0))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
+        }
+        for (int s0 = 0; prep && s0 < p->sys_count[b]; s0 += 65535)
+            if ((e = launch_prep(p->bucket_ids[b], p->max_nstep[b], std::min(65535, p->sys_count[b] - s0), bs,
+                                 p->d_sys, p->d_syslists + p->sys_begin[b] + s0)))
+                return set_err(MGPU_ERR_CUDA, "launching ldmd_prep_kernel", e);
+        if ((phases & 2) && jobs &&
+            (e = launch_prop(p->iprop, p->bucket_ids[b], p->job_count[b], p->smem[b], p->vl_smem[b], bs, p->d_sys,
                              p->d_jobs + p->job_begin[b], y_dev, nodes_dev, status_dev, kfail_dev)))
             return set_err(MGPU_ERR_CUDA, "launching the propagation kernel", e);
+        if (side >= 0 && (e = cudaEventRecord(p->sstreams[side].done, bs)))
+            return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     }
-    // the caller's stream waits for every large-N bucket
+    // the caller's stream waits for every bucket
+    for (size_t i = 0; fork && i < p->sstreams.size(); ++i)
+        if ((e = cudaStreamWaitEvent(st, p->sstreams[i].done, 0))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     for (size_t i = 0; i < p->big.size(); ++i)
         if ((e = cudaStreamWaitEvent(st, p->bstreams[i].done, 0)))
             return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
