@@ -24,7 +24,13 @@ namespace smx {
 
 constexpr int kMaxNShared = 64;  // matrices in shared memory up to here
 constexpr int kMaxN = 1024;       // global-memory scratch above
-constexpr int kThreads = 128;
+constexpr int kThreads = 128;     // of a job in shared memory
+// of a job in the global scratch: its matrices come from L2 once a pivot, so an
+// SM needs the loads of a whole block of warps in flight (128 threads and a
+// division per element: 43 ms for 48 jobs each of N = 72, 90, 128 and 199;
+// 1024 threads, a warp a row: see gauss_jordan)
+constexpr int kThreadsG = 1024;
+constexpr size_t kSmemG = 224 * 1024;  // dynamic shared memory of such a CTA at most
 // the matrices: [KM | T] with padded rows, then K (doubles)
 __host__ __device__ constexpr size_t mat_doubles(int n, int no) { return (size_t)n * (n + no + 1) + (size_t)no * no; }
 __host__ __device__ constexpr size_t smem_bytes(int n, int no) { return mat_doubles(n, no) * 8; }
@@ -115,7 +121,10 @@ __device__ double klogd(int l, double x)
 
 // Gauss-Jordan on the first `nr` rows of A (row stride lda): columns [0, nr)
 // are reduced to I, columns [nr, ncol) become A^{-1} B.  Partial pivoting when
-// `pivot`.  Returns false (all threads) on a zero pivot.
+// `pivot`.  Returns false (all threads) on a zero pivot.  The update of a pivot
+// takes the columns in groups of 32 CW, the pivot row's values of a group in
+// registers, and a warp to a row.
+template <int T, int CW>
 __device__ bool gauss_jordan(double *A, int lda, int nr, int ncol, bool pivot, int *s_p, double *s_f)
 {
     const int tid = threadIdx.x;
@@ -143,7 +152,7 @@ __device__ bool gauss_jordan(double *A, int lda, int nr, int ncol, bool pivot, i
         __syncthreads();
         const int p = pivot ? *s_p : k;
         if (p != k)
-            for (int j = tid; j < ncol; j += kThreads) {
+            for (int j = tid; j < ncol; j += T) {
                 const double t = A[k * lda + j];
                 A[k * lda + j] = A[p * lda + j];
                 A[p * lda + j] = t;
@@ -152,16 +161,29 @@ __device__ bool gauss_jordan(double *A, int lda, int nr, int ncol, bool pivot, i
         const double piv = A[k * lda + k];
         if (piv == 0.0 || !isfinite(piv)) return false;
         const double rp = 1.0 / piv;
-        for (int j = k + 1 + tid; j < ncol; j += kThreads) A[k * lda + j] *= rp;
-        for (int i = tid; i < nr; i += kThreads) s_f[i] = A[i * lda + k];
+        for (int j = k + 1 + tid; j < ncol; j += T) A[k * lda + j] *= rp;
+        for (int i = tid; i < nr; i += T) s_f[i] = A[i * lda + k];
         __syncthreads();
         if (tid == 0) A[k * lda + k] = 1.0;
-        const int w = ncol - k - 1;
-        for (int e = tid; e < nr * w; e += kThreads) {
-            const int i = e / w, j = k + 1 + e % w;
-            if (i != k) A[i * lda + j] = fma(-s_f[i], A[k * lda + j], A[i * lda + j]);
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int j0 = k + 1; j0 < ncol; j0 += 32 * CW) {
+            double row[CW];
+#pragma unroll
+            for (int c = 0; c < CW; ++c) {
+                const int j = j0 + 32 * c + lane;
+                row[c] = j < ncol ? A[(size_t)k * lda + j] : 0.0;
+            }
+#pragma unroll 2
+            for (int i = warp; i < nr; i += T / 32) {
+                if (i == k) continue;
+                const double f = -s_f[i];
+                double *ai = A + (size_t)i * lda + j0 + lane;
+#pragma unroll
+                for (int c = 0; c < CW; ++c)
+                    if (j0 + 32 * c + lane < ncol) ai[32 * c] = fma(f, row[c], ai[32 * c]);
+            }
         }
-        for (int i = tid; i < nr; i += kThreads)
+        for (int i = tid; i < nr; i += T)
             if (i != k) A[i * lda + k] = 0.0;
         __syncthreads();
     }
@@ -170,6 +192,7 @@ __device__ bool gauss_jordan(double *A, int lda, int nr, int ncol, bool pivot, i
 
 // One job: channel functions, [KM | T], Gauss-Jordan, K, then S.  A and K
 // point at shared or global memory; the channel arrays at shared memory.
+template <int T, int CW>
 __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restrict__ nb_all,
                             const int *__restrict__ nb_off, const double *__restrict__ y, double *__restrict__ sr,
                             double *__restrict__ si, int *__restrict__ status, double *A, double *K, double *sj,
@@ -178,7 +201,7 @@ __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restr
     const int n = S.n, no = job.nopen, tid = threadIdx.x;
     const int lda = n + no + 1;
     const double R = job.rmatch;
-    for (int c = tid; c < n; c += kThreads) {
+    for (int c = tid; c < n; c += T) {
         s_nb[c] = nb_all[nb_off[job.sys] + c];
         const double dif = job.ered - job.eint[c];
         const double w = copysign(sqrt(fabs(dif)), dif);
@@ -200,7 +223,7 @@ __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restr
     }
     __syncthreads();
     const double *yj = y + job.yoff;
-    for (int e = tid; e < n * (n + no); e += kThreads) {
+    for (int e = tid; e < n * (n + no); e += T) {
         const int i = e / (n + no), j = e % (n + no);
         const int a = s_nb[i];
         if (j < n) {
@@ -212,16 +235,16 @@ __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restr
         }
     }
     __syncthreads();
-    bool ok = gauss_jordan(A, lda, n, n + no, true, s_p, s_f);
+    bool ok = gauss_jordan<T, CW>(A, lda, n, n + no, true, s_p, s_f);
     // K = symmetrised open block of KM^{-1} T
     if (ok) {
-        for (int e = tid; e < no * no; e += kThreads) {
+        for (int e = tid; e < no * no; e += T) {
             const int i = e / no, j = e % no;
             K[i * no + j] = 0.5 * (A[i * lda + n + j] + A[j * lda + n + i]);
         }
         __syncthreads();
         // [0.5 K K + 0.5 I | I] in the first `no` rows of A, then Gauss-Jordan (I + K^2 is positive definite)
-        for (int e = tid; e < no * 2 * no; e += kThreads) {
+        for (int e = tid; e < no * 2 * no; e += T) {
             const int i = e / (2 * no), j = e % (2 * no);
             double v;
             if (j < no) {
@@ -234,7 +257,7 @@ __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restr
             A[i * lda + j] = v;
         }
         __syncthreads();
-        ok = gauss_jordan(A, lda, no, 2 * no, false, s_p, s_f);
+        ok = gauss_jordan<T, CW>(A, lda, no, 2 * no, false, s_p, s_f);
     }
     if (!ok) {
         if (tid == 0) status[job.out] = MGPU_ERR_INVERSION;
@@ -242,7 +265,7 @@ __device__ void smatrix_job(const SysDev &S, const SJob &job, const int *__restr
     }
     // SR = SRINV - I, SI = SRINV K (column-major, channel order NB)
     double *srj = sr + job.soff, *sij = si + job.soff;
-    for (int e = tid; e < no * no; e += kThreads) {
+    for (int e = tid; e < no * no; e += T) {
         const int i = e % no, j = e / no;
         const double inv = A[i * lda + no + j];
         double v = 0.0;
@@ -266,15 +289,17 @@ smatrix_kernel(const SysDev *__restrict__ systems, const SJob *__restrict__ jobs
     if (status[job.out] != MGPU_OK || job.nopen == 0) return;  // the propagation failed, or no open channel: no S
     double *A = smx_sm;                                          // n x (n + no): [KM | T]
     double *K = smx_sm + (size_t)S.n * (S.n + job.nopen + 1);    // no x no
-    smatrix_job(S, job, nb_all, nb_off, y, sr, si, status, A, K, sj, sjp, sn, snp, s_f, s_nb, &s_p);
+    smatrix_job<kThreads, 2>(S, job, nb_all, nb_off, y, sr, si, status, A, K, sj, sjp, sn, snp, s_f, s_nb, &s_p);
 }
 
-// N <= 1024: the matrices in the global scratch at job.scr, the channel
-// arrays in shared memory (chan_smem_bytes)
-__global__ void __launch_bounds__(kThreads)
+// N <= 1024: the channel arrays in shared memory (chan_smem_bytes), the matrices
+// behind them (at double moff) where they fit its `room` doubles (up to about
+// N = 120), else in the global scratch at job.scr
+__global__ void __launch_bounds__(kThreadsG)
 smatrix_kernel_g(const SysDev *__restrict__ systems, const SJob *__restrict__ jobs, const int *__restrict__ nb_all,
                  const int *__restrict__ nb_off, const double *__restrict__ y, double *__restrict__ sr,
-                 double *__restrict__ si, int *__restrict__ status, double *__restrict__ scratch)
+                 double *__restrict__ si, int *__restrict__ status, double *__restrict__ scratch, unsigned moff,
+                 unsigned room)
 {
     extern __shared__ __align__(16) double smx_sm[];
     __shared__ int s_p;
@@ -284,9 +309,9 @@ smatrix_kernel_g(const SysDev *__restrict__ systems, const SJob *__restrict__ jo
     const int n = S.n;
     double *sj = smx_sm, *sjp = sj + n, *sn = sjp + n, *snp = sn + n, *s_f = snp + n;
     int *s_nb = reinterpret_cast<int *>(s_f + n);
-    double *A = scratch + job.scr;
+    double *A = mat_doubles(n, job.nopen) <= room ? smx_sm + moff : scratch + job.scr;
     double *K = A + (size_t)n * (n + job.nopen + 1);
-    smatrix_job(S, job, nb_all, nb_off, y, sr, si, status, A, K, sj, sjp, sn, snp, s_f, s_nb, &s_p);
+    smatrix_job<kThreadsG, 4>(S, job, nb_all, nb_off, y, sr, si, status, A, K, sj, sjp, sn, snp, s_f, s_nb, &s_p);
 }
 
 // YTRANS's transform (TRNSFM, ytrans.f90:410-413) Y' = EVEC^T Y EVEC for

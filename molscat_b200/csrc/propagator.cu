@@ -1050,6 +1050,7 @@ struct mgpu_plan {
     std::vector<size_t> soff;
     size_t selems = 0;
     size_t s_smem = 0, s_smem_g = 0;
+    size_t s_moff_g = 0, s_room_g = 0;     // of s_smem_g: where the matrices of the jobs that fit start, their room (doubles)
     int ns_small = 0, ns_large = 0;
     size_t sscr_elems = 0;
     double *d_sscr = nullptr;
@@ -1741,7 +1742,8 @@ static int build_s(mgpu_plan *p)
     std::vector<smx::SJob> sj, sjg;
     p->nopen.assign(njobs, 0);
     p->soff.assign(njobs, 0);
-    p->s_smem = p->s_smem_g = 0;
+    p->s_smem = p->s_smem_g = p->s_room_g = 0;
+    std::vector<size_t> mats;  // doubles of the larger jobs' matrices
     size_t so = 0, scr = 0;
     for (int j = 0; j < njobs; ++j) {
         const int sy = p->job_sys[j];
@@ -1774,10 +1776,17 @@ static int build_s(mgpu_plan *p)
                 scr += smx::mat_doubles(n, no);
             }
             p->s_smem_g = std::max(p->s_smem_g, smx::chan_smem_bytes(n));
+            if (no > 0) mats.push_back(smx::mat_doubles(n, no));
             sjg.push_back(q);
         }
     }
     p->selems = so;
+    // one CTA of the larger jobs' kernel fills an SM's threads, so it may take its shared memory too
+    p->s_moff_g = (p->s_smem_g + 15) / 16 * 2;
+    const size_t room = smx::kSmemG / sizeof(double) - std::min(smx::kSmemG / sizeof(double), p->s_moff_g);
+    for (size_t m : mats)
+        if (m <= room) p->s_room_g = std::max(p->s_room_g, m);
+    p->s_smem_g = (p->s_moff_g + p->s_room_g) * sizeof(double);
     if (scr != p->sscr_elems && p->d_sscr) {
         cudaFree(p->d_sscr);
         p->d_sscr = nullptr;
@@ -2286,8 +2295,9 @@ int mgpu_plan_smatrix_device(mgpu_plan *p, const double *y_dev, double *sr_dev, 
         if ((e = set_smem(smx::smatrix_kernel_g, p->s_smem_g)))
             return set_err(MGPU_ERR_CUDA, "S-matrix kernel set-up", e);
         for (int j0 = 0; j0 < p->ns_large; j0 += 65535) {
-            smx::smatrix_kernel_g<<<std::min(65535, p->ns_large - j0), smx::kThreads, p->s_smem_g, st>>>(
-                p->d_sys, p->d_sjobs_g + j0, p->d_nb, p->d_nb_off, y_dev, sr_dev, si_dev, status_dev, p->d_sscr);
+            smx::smatrix_kernel_g<<<std::min(65535, p->ns_large - j0), smx::kThreadsG, p->s_smem_g, st>>>(
+                p->d_sys, p->d_sjobs_g + j0, p->d_nb, p->d_nb_off, y_dev, sr_dev, si_dev, status_dev, p->d_sscr,
+                (unsigned)p->s_moff_g, (unsigned)p->s_room_g);
             if ((e = cudaGetLastError())) return set_err(MGPU_ERR_CUDA, "launching the S-matrix kernel", e);
         }
     }
