@@ -2812,13 +2812,8 @@ extern "C" int mgpu_ldma_run_host(mgpu_ldma *h, int njobs, const double *ered, d
         (e = cudaMemcpyAsync(dy, y, njobs * nn * sizeof(double), cudaMemcpyHostToDevice, st)))
         rc = set_err(MGPU_ERR_CUDA, "copying LDMA inputs", e);
     if (!rc) {
-        const size_t sm = mgpu::ldma::smem_bytes(h->t.n);
-        if ((e = set_smem(mgpu::ldma::ldma_kernel, sm))) {
-            rc = set_err(MGPU_ERR_CUDA, "ldma_kernel set-up", e);
-        } else {
-            mgpu::ldma::ldma_kernel<<<njobs, mgpu::ldma::kThreads, sm, st>>>(h->t, de, dy, dn, ds);
-            if ((e = cudaGetLastError())) rc = set_err(MGPU_ERR_CUDA, "launching ldma_kernel", e);
-        }
+        if ((e = mgpu::ldma::launch_ldma(h->t, njobs, de, dy, dn, ds, st)))
+            rc = set_err(MGPU_ERR_CUDA, "launching ldma_kernel", e);
     }
     if (!rc && ((e = cudaMemcpyAsync(y, dy, njobs * nn * sizeof(double), cudaMemcpyDeviceToHost, st)) ||
                 (e = cudaMemcpyAsync(nodes, dn, njobs * sizeof(int), cudaMemcpyDeviceToHost, st)) ||
@@ -2897,13 +2892,8 @@ extern "C" int mgpu_airy_run_host(mgpu_airy *h, int njobs, const double *y124, d
         (e = cudaMemcpyAsync(dz, z, njobs * nn * sizeof(double), cudaMemcpyHostToDevice, st)))
         rc = set_err(MGPU_ERR_CUDA, "copying AIRY inputs", e);
     if (!rc) {
-        const size_t sm = mgpu::ldma::smem_bytes(h->t.n);
-        if ((e = set_smem(mgpu::ldma::airy_kernel, sm))) {
-            rc = set_err(MGPU_ERR_CUDA, "airy_kernel set-up", e);
-        } else {
-            mgpu::ldma::airy_kernel<<<njobs, mgpu::ldma::kThreads, sm, st>>>(h->t, dy, dz, dn, ds);
-            if ((e = cudaGetLastError())) rc = set_err(MGPU_ERR_CUDA, "launching airy_kernel", e);
-        }
+        if ((e = mgpu::ldma::launch_airy(h->t, njobs, dy, dz, dn, ds, st)))
+            rc = set_err(MGPU_ERR_CUDA, "launching airy_kernel", e);
     }
     if (!rc && ((e = cudaMemcpyAsync(z, dz, njobs * nn * sizeof(double), cudaMemcpyDeviceToHost, st)) ||
                 (e = cudaMemcpyAsync(nodes, dn, njobs * sizeof(int), cudaMemcpyDeviceToHost, st)) ||
