@@ -38,11 +38,8 @@ using wf::tix;
 constexpr int NB = 64;      // pivots per round
 constexpr int KB = NB / 8;  // tile columns per round
 constexpr int MC = NB / 4;  // m8n8k4 k-steps per round
-// Factor CTA sizes: a whole SM's registers (1024 threads at 64) where the
-// update beside it is small (NT <= FACT_BIG_MAX_NT), half of them above.
-constexpr int FACT_THREADS = 512;
-constexpr int FACT_THREADS_BIG = 1024;
-constexpr int FACT_BIG_MAX_NT = 32;
+// Up to this NT a round's diagonal-block update stays on the main stream.
+constexpr int DIAG_MAIN_MAX_NT = 32;
 constexpr int PANEL_WARPS = 8;
 #ifndef MGPU_UPD_WARPS
 #define MGPU_UPD_WARPS 4
@@ -118,191 +115,164 @@ __device__ __forceinline__ void report_failure(const MatDesc &md, int flags, int
 
 // ---------------------------------------------------------------------------
 // factor: LDL^T of the 64x64 pivot block, Lam = L^{-1}, 1/delta
-// Sixteen sub-blocks of four pivots (the 4-pivot step of warp_dmma.cuh).  For
-// sub-block p: rows below form c = Lam4 D[i, p..p+3]; the trailing lower part
-// of D and the rows of Lam below take the rank-4 updates
-//     D_ij -= sum_m c_m(i) c_m(j)/delta_m ,  Lam_i -= sum_m (c_m(i)/delta_m) Lam_p+m
-// (elimination applied to I).  Look-ahead: warp 0 owns no trailing element;
-// while the other warps update, it updates the next 4x4 diagonal block first
-// and factors it (ldl_block4), so the chain of pivot reciprocals overlaps the
-// rank-4 updates.
+// Eight pivots at a time, with the pieces of the one-CTA sweep
+// (kernels_cta.cuh).  For the 8x8 diagonal block K, factored as two blocks of
+// four pivots (cta::factor8):
+//   1. row i below it: operands c1, x1 = -c1/delta, c2, x2 (the update of its
+//      P2 entries by P1 between them); beside that, the rows of Lam at the
+//      block: Lam_P1 = Lam1 Lam_P1, Lam_P2 += X1(P2) Lam_P1, Lam_P2 = Lam2 Lam_P2,
+//      a thread to a column;                                       barrier
+//   2. the trailing tiles D_IJ += X_I c_J and the tiles of Lam below,
+//      Lam_IM += X_I Lam_KM (elimination applied to I), two DMMAs each; the last
+//      warp does the next diagonal tile first and factors it.       barrier
+// It is the latency chain of a round (one CTA a matrix): 64 pivots one after the
+// other in sixteen four-pivot steps with element updates between barriers took
+// 29 us at N = 500 x 48 (N = 500, 48 energies: 11.6 -> 14.3 TFLOP/s with this form,
+// N = 256 4.6 -> 6.1, N = 1000, update-bound, 19.9 -> 20.3).
 // ---------------------------------------------------------------------------
-constexpr size_t kFactSmem = 2 * (size_t)NB * (NB + 1) * sizeof(double);  // D and Lam, padded rows
-// element ownership in a factor CTA of T threads (warp 0 factors the sub-blocks)
-template <int T>
-struct FactShape {
-    static_assert(T >= 5 * NB && T % 32 == 0, "factor CTA: 4 NB rows of c(i) and every Lam column at once");
-    static constexpr int own = T - 32;                                   // threads owning elements
-    static constexpr int d = (NB * (NB + 1) / 2 + own - 1) / own;        // D elements per thread
-    static constexpr int l = (NB * (NB - 1) / 2 + own - 1) / own;        // Lam elements per thread
+constexpr int FACT_WARPS = 8;
+constexpr int FACT_THREADS = 32 * FACT_WARPS;
+constexpr int FP = NB + 8;      // row pitch of D and Lam: a tile's rows on distinct bank groups
+constexpr int FLD = NB + 2;     // column pitch of the operands (pairs), as in kernels_cta.cuh
+struct FactSm {
+    static constexpr int D = 0;                          // [64][FP] lower triangle
+    static constexpr int L = D + NB * FP;                // [64][FP] Lam
+    static constexpr int XS = L + NB * FP;               // X operands [4][FLD] pairs (P1, P2)
+    static constexpr int BS = XS + 8 * FLD;              // c operands
+    static constexpr int DT = BS + 8 * FLD;              // the diagonal tile being factored
+    static constexpr int FB = DT + 64;                   // cta::Fact, twice (parity of K)
+    static constexpr int RD = FB + 2 * cta::Fact::SIZE;  // 1/delta
+    static constexpr int SIZE = RD + NB;
 };
+constexpr size_t kFactSmem = (size_t)FactSm::SIZE * sizeof(double);
 
-__device__ __forceinline__ void tri_rc(int e, int &i, int &j)  // e -> (i, j), j <= i
-{
-    int r = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
-    while (r * (r + 1) / 2 > e) --r;
-    while ((r + 1) * (r + 2) / 2 <= e) ++r;
-    i = r;
-    j = e - r * (r + 1) / 2;
-}
-
-template <int T>
-__global__ void __launch_bounds__(T)
+__global__ void __launch_bounds__(FACT_THREADS)
 big_factor_kernel(const MatDesc *__restrict__ mds, Panels pn, int round, const int *__restrict__ kstep)
 {
-    constexpr int kFactOwn = FactShape<T>::own, kFactD = FactShape<T>::d, kFactL = FactShape<T>::l;
     extern __shared__ __align__(16) double fsm[];
-    double (*D)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(fsm);
-    double (*L)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(fsm + NB * (NB + 1));
-    __shared__ __align__(16) double s_c[NB][4];  // c(i) of the current sub-block
-    __shared__ __align__(16) double s_t[NB][4];  // c(i) / delta
-    __shared__ double s_f[16];                   // ldl_block4 operands of the current sub-block
-    __shared__ double s_r[NB];
-    __shared__ int s_cnt, s_flags;
     const MatDesc md = mds[blockIdx.x];
     const int k = *kstep;
     if (k > md.nstep) return;
+    double *D = fsm + FactSm::D, *L = fsm + FactSm::L, *dt = fsm + FactSm::DT, *rd = fsm + FactSm::RD;
+    double2 *xs = reinterpret_cast<double2 *>(fsm + FactSm::XS), *bs = reinterpret_cast<double2 *>(fsm + FactSm::BS);
     const int p0 = NB * round, K0 = KB * round;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) s_cnt = s_flags = 0;
-    for (int x = tid; x < NB * NB; x += T) {
-        const int i = x >> 6, j = x & 63;
-        double v = 0.0;
-        if (j <= i) v = md.a[(size_t)tix(K0 + (i >> 3), K0 + (j >> 3)) * 64 + ((i & 7) * 4 + ((j & 7) >> 1)) * 2 + (j & 1)];
-        D[i][j] = v;
-        L[i][j] = (i == j) ? 1.0 : 0.0;
-    }
-    // owned elements (packed (i << 8) | j, -1 when none): D lower triangle, Lam strictly lower
-    int od[kFactD], ol[kFactL];
-#pragma unroll
-    for (int u = 0; u < kFactD; ++u) {
-        const int e = (tid - 32) + u * kFactOwn;
-        int i = 0, j = 0;
-        const bool ok = warp > 0 && e < NB * (NB + 1) / 2;
-        if (ok) tri_rc(e, i, j);
-        od[u] = ok ? ((i << 8) | j) : -1;
-    }
-#pragma unroll
-    for (int u = 0; u < kFactL; ++u) {
-        const int e = (tid - 32) + u * kFactOwn;
-        int i = 0, c = 0;
-        const bool ok = warp > 0 && e < NB * (NB - 1) / 2;
-        if (ok) tri_rc(e, i, c);
-        ol[u] = ok ? (((i + 1) << 8) | c) : -1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, q = lane & 3;
+    const bool factoring = warp == FACT_WARPS - 1;
+    // the lower tiles of D, a warp a tile; the padding takes unit pivots; Lam = I
+    for (int t = warp; t < KB * (KB + 1) / 2; t += FACT_WARPS) {
+        int I, J;
+        tile_ij(t, I, J);
+        double2 v = *reinterpret_cast<const double2 *>(md.a + (size_t)tix(K0 + I, K0 + J) * 64 + lane * 2);
+        const int i = 8 * I + r, j = 8 * J + 2 * q;
+        if (p0 + i >= md.n) {
+            if (i == j) v.x = 1.0;
+            if (i == j + 1) v.y = 1.0;
+        }
+        *reinterpret_cast<double2 *>(D + i * FP + j) = v;
+        *reinterpret_cast<double2 *>(L + i * FP + j) = make_double2(i == j ? 1.0 : 0.0, i == j + 1 ? 1.0 : 0.0);
     }
     __syncthreads();
-    // warp 0 factors one 4x4 diagonal sub-block (rows q..q+3 of D final)
-    auto sub_factor = [&](int q) {
-        double f[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j <= i; ++j) f[i][j] = D[q + i][q + j];
-        int cnt = 0, flags = 0;
-        wf::ldl_block4(f, md.n - p0 - q, cnt, flags);
-        if (lane == 0) {
-            s_cnt += cnt;
-            s_flags |= flags;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) s_f[i * 4 + j] = f[i][j];
-        }
+    int cnt = 0, flags = 0;
+    // diagonal tile K to dt (rows eight apart) and its factors
+    auto factor_tile = [&](int K, double2 v) {
+        *reinterpret_cast<double2 *>(dt + r * 8 + 2 * q) = v;
+        double *fb = fsm + FactSm::FB + (K & 1) * cta::Fact::SIZE;
+        cta::factor8(dt, fb, lane, cnt, flags);
+        __syncwarp();
+        if (lane < 8) rd[8 * K + lane] = fb[(lane < 4 ? cta::Fact::P1 : cta::Fact::P2) + (lane & 3)];
     };
-    if (warp == 0) sub_factor(0);
-    for (int sb = 0; sb < NB / 4; ++sb) {
-        const int p = 4 * sb;
-        __syncthreads();
-        double f[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) f[i][j] = s_f[i * 4 + j];
-        if (tid < 4) s_r[p + tid] = (tid == 0) ? f[0][0] : (tid == 1) ? f[1][1] : (tid == 2) ? f[2][2] : f[3][3];
-        // c(i) = Lam4 D[i, p..p+3] for rows below; Lam rows of the sub-block = Lam4 Lam_sub
-        if (tid < 4 * NB) {
-            const int i = tid >> 2, m = tid & 3;
-            if (i >= p + 4) {
-                double lq[3], rq;
-                wf::lane_operands(f, m, lq, rq);  // row m of Lam4 below the diagonal, 1/delta_m
-                const double c = fma(lq[0], D[i][p], fma(lq[1], D[i][p + 1], fma(lq[2], D[i][p + 2], D[i][p + m])));
-                s_c[i][m] = c;
-                s_t[i][m] = c * rq;
-            }
-        } else {
-            // one column per thread, in place from the last row up (row m reads the old rows above it)
-            const int c = tid - 4 * NB;
-            if (c < p + 4) {
-#pragma unroll
-                for (int m = 3; m >= 1; --m) {
-                    double v = L[p + m][c];
-#pragma unroll
-                    for (int mm = 0; mm < 3; ++mm)
-                        if (mm < m) v = fma(f[m][mm], L[p + mm][c], v);
-                    L[p + m][c] = v;
-                }
-            }
-        }
-        __syncthreads();
-        const int q = p + 4;  // next sub-block
-        if (warp == 0) {
-            if (q < NB) {
-                if (lane < 10) {
-                    int ii, jj;
-                    tri_rc(lane, ii, jj);
-                    const int i = q + ii, j = q + jj;
-                    double v = D[i][j];
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) v = fma(-s_t[i][m], s_c[j][m], v);
-                    D[i][j] = v;
-                }
-                __syncwarp();
-                sub_factor(q);
-            }
-        } else {
-#pragma unroll
-            for (int u = 0; u < kFactD; ++u) {
-                const int i = od[u] >> 8, j = od[u] & 255;
-                if (od[u] >= 0 && j >= q && !(i < q + 4)) {  // the next diagonal block is warp 0's
-                    const double2 t01 = *reinterpret_cast<const double2 *>(&s_t[i][0]);
-                    const double2 t23 = *reinterpret_cast<const double2 *>(&s_t[i][2]);
-                    const double2 c01 = *reinterpret_cast<const double2 *>(&s_c[j][0]);
-                    const double2 c23 = *reinterpret_cast<const double2 *>(&s_c[j][2]);
-                    double v = D[i][j];
-                    v = fma(-t01.x, c01.x, v);
-                    v = fma(-t01.y, c01.y, v);
-                    v = fma(-t23.x, c23.x, v);
-                    v = fma(-t23.y, c23.y, v);
-                    D[i][j] = v;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kFactL; ++u) {
-                const int i = ol[u] >> 8, c = ol[u] & 255;
-                if (ol[u] >= 0 && i >= q && c < q) {
-                    const double2 t01 = *reinterpret_cast<const double2 *>(&s_t[i][0]);
-                    const double2 t23 = *reinterpret_cast<const double2 *>(&s_t[i][2]);
-                    double v = L[i][c];
-                    v = fma(-t01.x, L[p][c], v);
-                    v = fma(-t01.y, L[p + 1][c], v);
-                    v = fma(-t23.x, L[p + 2][c], v);
-                    v = fma(-t23.y, L[p + 3][c], v);
-                    L[i][c] = v;
-                }
-            }
-        }
-    }
+    if (factoring) factor_tile(0, *reinterpret_cast<const double2 *>(D + r * FP + 2 * q));
     __syncthreads();
-    // Lam in the panel's B-fragment order: (row 8kt + ln/4, column 4mc + ln%4) at (kt MC + mc) 32 + ln
-    double *lam = pn.lam + (size_t)blockIdx.x * NB * NB;
-    for (int x = tid; x < NB * NB; x += T) {
-        const int ln = x & 31, mc = (x >> 5) % MC, kt = x / (32 * MC);
-        lam[x] = L[8 * kt + (ln >> 2)][4 * mc + (ln & 3)];
+#pragma unroll 1
+    for (int K = 0; K < KB; ++K) {
+        const double *f = fsm + FactSm::FB + (K & 1) * cta::Fact::SIZE;
+        const int below = NB - 8 * (K + 1);  // rows below the block
+        // 1. a thread to a row below, and (the upper warps) to a column of Lam
+        if (tid < below) {
+            const int i = 8 * (K + 1) + tid;
+            const double2 *row = reinterpret_cast<const double2 *>(D + i * FP + 8 * K);
+            const double2 t0 = row[0], t1 = row[1], t2 = row[2], t3 = row[3];
+            const double v[4] = {t0.x, t0.y, t1.x, t1.y};
+            double w[4] = {t2.x, t2.y, t3.x, t3.y}, c1[4], x1[4], c2[4], x2[4];
+            wf::Block4 b;
+            cta::get_block4(f + cta::Fact::P1, b);
+            cta::row_operands(b, v, c1, x1);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) w[m] = fma(x1[kk], f[cta::Fact::C + 4 * m + kk], w[m]);
+            cta::get_block4(f + cta::Fact::P2, b);
+            cta::row_operands(b, w, c2, x2);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                xs[kk * FLD + i] = make_double2(x1[kk], x2[kk]);
+                bs[kk * FLD + i] = make_double2(c1[kk], c2[kk]);
+            }
+        } else if (tid >= 64 && tid - 64 < 8 * (K + 1)) {
+            double *col = L + 8 * K * FP + tid - 64, v[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = col[m * FP];
+            wf::Block4 b;
+            auto apply = [&](double *u) {  // u = Lam4 u, the last row first
+                u[3] = fma(b.m32, u[2], fma(b.m31, u[1], fma(b.m30, u[0], u[3])));
+                u[2] = fma(b.m21, u[1], fma(b.m20, u[0], u[2]));
+                u[1] = fma(b.m10, u[0], u[1]);
+            };
+            cta::get_block4(f + cta::Fact::P1, b);
+            apply(v);
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) v[4 + m] = fma(f[cta::Fact::X + 4 * m + kk], v[kk], v[4 + m]);
+            cta::get_block4(f + cta::Fact::P2, b);
+            apply(v + 4);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) col[m * FP] = v[m];
+        }
+        __syncthreads();
+        if (K + 1 == KB) break;
+        // 2. the tiles: D(I, J), J > K, in row order behind the next diagonal one, then Lam(I, M), M <= K
+        auto update = [&](double *c, int I, double2 b) {
+            const double2 x = xs[q * FLD + 8 * I + r];
+            double2 v = *reinterpret_cast<const double2 *>(c + r * FP + 2 * q);
+            wf::dmma(v.x, v.y, x.x, b.x);
+            wf::dmma(v.x, v.y, x.y, b.y);
+            *reinterpret_cast<double2 *>(c + r * FP + 2 * q) = v;
+            return v;
+        };
+        const int nr = KB - K - 1, nd = nr * (nr + 1) / 2;  // tile rows below, trailing tiles of D
+        if (factoring) {
+            const double2 v = update(D + 8 * (K + 1) * FP + 8 * (K + 1), K + 1, bs[q * FLD + 8 * (K + 1) + r]);
+            factor_tile(K + 1, v);
+        } else {
+            for (int t = 1 + warp; t < nd + nr * (K + 1); t += FACT_WARPS - 1) {
+                int I, J;
+                if (t < nd) {
+                    tile_ij(t, I, J);
+                    I += K + 1;
+                    J += K + 1;
+                    update(D + 8 * I * FP + 8 * J, I, bs[q * FLD + 8 * J + r]);
+                } else {
+                    I = K + 1 + (t - nd) / (K + 1);
+                    J = (t - nd) % (K + 1);
+                    const double *row = L + (8 * K + q) * FP + 8 * J + r;
+                    update(L + 8 * I * FP + 8 * J, I, make_double2(row[0], row[4 * FP]));
+                }
+            }
+        }
+        __syncthreads();
     }
-    if (tid < NB) pn.rd[(size_t)blockIdx.x * NB + tid] = s_r[tid];
-    if (tid == 0) {
-        if (s_cnt) atomicAdd(md.cnt, md.sign * s_cnt);
-        if (s_flags) report_failure(md, s_flags, k);
+    // Lam in the panel's B-fragment order: (row 8kt + ln/4, column 4mc + ln%4) at (kt MC + mc) 32 + ln; the
+    // panel's k-steps read the blocks up to the diagonal only
+    double *lam = pn.lam + (size_t)blockIdx.x * NB * NB;
+    for (int x = tid; x < NB * NB; x += FACT_THREADS) {
+        const int ln = x & 31, mc = (x >> 5) % MC, kt = x / (32 * MC), i = 8 * kt + (ln >> 2), j = 4 * mc + (ln & 3);
+        lam[x] = j <= i ? L[i * FP + j] : 0.0;
+    }
+    if (tid < NB) pn.rd[(size_t)blockIdx.x * NB + tid] = rd[tid];
+    if (factoring && lane == 0) {
+        if (cnt) atomicAdd(md.cnt, md.sign * cnt);
+        if (flags) report_failure(md, flags, k);
     }
 }
 

@@ -1194,13 +1194,10 @@ static cudaError_t big_invert(const big::MatDesc *md, int M, int nt, const big::
         gcol(big::UPD_SPLIT * (nbk - 1), M), gdiag(big::UPD_SPLIT, M);
     const int ut = 32 * big::UPD_WARPS, pt = 32 * big::PANEL_WARPS;
     cudaStream_t side = ax.side;
-    const bool diag_side = nt > big::FACT_BIG_MAX_NT;
+    const bool diag_side = nt > big::DIAG_MAIN_MAX_NT;
     cudaError_t e;
     auto factor = [&](const big::Panels &p, int R, cudaStream_t s) {
-        if (nt <= big::FACT_BIG_MAX_NT)
-            big::big_factor_kernel<big::FACT_THREADS_BIG><<<M, big::FACT_THREADS_BIG, big::kFactSmem, s>>>(md, p, R, kstep);
-        else
-            big::big_factor_kernel<big::FACT_THREADS><<<M, big::FACT_THREADS, big::kFactSmem, s>>>(md, p, R, kstep);
+        big::big_factor_kernel<<<M, big::FACT_THREADS, big::kFactSmem, s>>>(md, p, R, kstep);
     };
     factor(pn[0], 0, st);
     big::big_panel_kernel<<<gp, pt, 0, st>>>(md, pn[0], nt, 0, kstep);
@@ -1508,8 +1505,7 @@ static cudaError_t run_big_prop(BigBucket &g, int iprop, const SysDev *d_sys, do
 static cudaError_t big_kernel_attributes()
 {
     cudaError_t e;
-    if ((e = set_smem(big::big_update_kernel, big::kUpdSmem)) || (e = set_smem(big::big_factor_kernel<big::FACT_THREADS>, big::kFactSmem)) ||
-        (e = set_smem(big::big_factor_kernel<big::FACT_THREADS_BIG>, big::kFactSmem)))
+    if ((e = set_smem(big::big_update_kernel, big::kUpdSmem)) || (e = set_smem(big::big_factor_kernel, big::kFactSmem)))
         return e;
     return cudaSuccess;
 }
