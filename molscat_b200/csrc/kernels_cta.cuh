@@ -45,7 +45,20 @@ struct CG {
     static constexpr int NPAD = 8 * NT;
     static constexpr int NTHR = 32 * W;
     static constexpr int TW = W - 1;                                // tile warps
-    static constexpr int TPW = (NT * (NT - 1) / 2 + TW - 1) / TW;   // tile slots of one of them
+    // The factoring warp's chain of DFMAs waits for the DMMAs of the other warps on its
+    // scheduler's FP64 pipe.  At NT = 14 and 20 those warps (3, 7, .. of 4n) take LN / LDEN of
+    // the others' tiles: LDMD, 1184 jobs, N = 106 6.87 -> 7.37 TFLOP/s, N = 150 6.91 -> 7.23
+    // (48 jobs 2.25 -> 2.34).  Elsewhere it costs a tile slot or gives nothing: N = 128
+    // 8.50 -> 8.29, N = 199 7.70 -> 7.40, N = 72 on four warps has no such warp.
+    static constexpr int LIGHT = NT == 14 || NT == 20 ? TW / 4 : 0;
+    static constexpr int LN = W <= 8 ? 2 : 4, LDEN = W <= 8 ? 3 : 5;
+    // tiles of one of the other warps when there are `ntiles` off the diagonal
+    __host__ __device__ static constexpr int heavy(int ntiles)
+    {
+        const int parts = LDEN * (TW - LIGHT) + LN * LIGHT;
+        return (LDEN * ntiles + parts - 1) / parts;
+    }
+    static constexpr int TPW = heavy(NT * (NT - 1) / 2);            // tile slots of a warp
     static constexpr int TD = NTL * 64;                             // doubles of one tiled matrix
     // pitch of the panel and operand columns in 16-byte pairs: 2 mod 8, so that the
     // eight lanes of an access phase meet eight bank groups; eight rows past the
@@ -92,9 +105,10 @@ struct Own {
         warp = threadIdx.x >> 5;
         lane = threadIdx.x & 31;
         nb = (n + 7) >> 3;
-        const int nact = nb * (nb - 1) / 2, per = (nact + C::TW - 1) / C::TW;
-        e0 = warp * per;
-        ntw = warp < C::TW ? max(0, min(per, nact - e0)) : 0;
+        const int nact = nb * (nb - 1) / 2, hv = C::heavy(nact);
+        const int lt = C::LIGHT ? max(0, nact - (C::TW - C::LIGHT) * hv + C::LIGHT - 1) / max(1, C::LIGHT) : hv;
+        e0 = (warp - warp / 4) * hv + warp / 4 * lt;
+        ntw = warp < C::TW ? max(0, min(C::LIGHT && (warp & 3) == 3 ? lt : hv, nact - e0)) : 0;
         dg = sm + CSmem<NT, W>::DG;
 #pragma unroll
         for (int u = 0; u < C::TPW; ++u) {
