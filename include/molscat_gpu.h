@@ -168,9 +168,11 @@ int mgpu_plan_run_host(mgpu_plan *plan, double *y, int *nodes, int *status, int 
 /* Device buffers (y_dev in/out, nodes_dev/status_dev/kfail_dev out) on the
  * given cudaStream_t passed as void* (NULL = legacy default stream).
  * Asynchronous: returns after the launches are queued.  Each large-N bucket
- * runs on a stream pair of the plan's own, forked from and joined back into
- * `stream`, so buckets of different N overlap; the stream must therefore not
- * be capturing a graph. */
+ * runs on a stream pair of the plan's own and each small-N bucket after the
+ * first on a stream of its own, forked from and joined back into `stream`, so
+ * buckets of different N overlap.  After an error `stream` is ordered behind
+ * whatever was queued before it, too.  `stream` may be capturing a graph if
+ * the plan has no large-N bucket (the others then run in turn on it). */
 int mgpu_plan_run_device(mgpu_plan *plan, double *y_dev, int *nodes_dev,
                          int *status_dev, int *kfail_dev, void *stream);
 

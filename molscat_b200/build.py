@@ -16,7 +16,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libmolscat_gpu.so")
 SOURCES = [os.path.join(PKG, "csrc", "propagator.cu")]
-DEPS = SOURCES + sorted(glob.glob(os.path.join(PKG, "csrc", "*.cuh"))) + [os.path.join(ROOT, "include", "molscat_gpu.h")]
+DEPS = SOURCES + sorted(glob.glob(os.path.join(PKG, "csrc", "*.cuh")) + glob.glob(os.path.join(PKG, "csrc", "*.h"))) + [os.path.join(ROOT, "include", "molscat_gpu.h")]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17",

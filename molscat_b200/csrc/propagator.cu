@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "molscat_gpu.h"
+#include "stream_fork.h"
 #include "tiles.cuh"
 
 namespace mgpu {
@@ -673,6 +674,7 @@ static const Bucket kBuckets[] = {
 #undef X
 };
 static const int kNumBuckets = sizeof(kBuckets) / sizeof(kBuckets[0]);
+static_assert(sizeof(kBuckets) / sizeof(kBuckets[0]) <= StreamFork::kMaxSides, "a run forks at most a stream a bucket");
 
 static bool frag_layout(int b) { return kBuckets[b].kind != KIND_TILE4; }
 // 0 = 4x4 register tiles, 1 = 8x8 DMMA fragments, 2 = the same with the one-warp
@@ -2098,22 +2100,20 @@ int mgpu_plan_run_device_phases(mgpu_plan *p, double *y_dev, int *nodes_dev, int
     // A caller capturing a graph gets the small-N buckets one after the other on its own stream.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!p->sstreams.empty() && (e = cudaStreamIsCapturing(st, &cap))) return set_err(MGPU_ERR_CUDA, "stream state", e);
-    const bool fork = !p->sstreams.empty() && cap == cudaStreamCaptureStatusNone;
-    if (fork || !p->big.empty()) {
-        // the buckets' own streams are ordered after the caller's
-        if ((e = cudaEventRecord(p->ev_in, st))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
-    }
+    const bool own_streams = !p->sstreams.empty() && cap == cudaStreamCaptureStatusNone;
+    // the buckets' own streams are ordered after the caller's, and the caller's after them on every way out
+    StreamFork fork(st, p->ev_in);
+    if ((own_streams || !p->big.empty()) && (e = fork.begin())) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     // every large-N bucket on its own stream pair
     for (size_t i = 0; i < p->big.size(); ++i) {
         BigBucket &g = p->big[i];
         const mgpu_plan::BigStreams &q = p->bstreams[i];
-        if ((e = cudaStreamWaitEvent(q.st, p->ev_in, 0))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
+        if ((e = fork.to(q.st, q.done, q.side, q.evj))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
         if (prep && (e = run_big_prep(g, p->d_sys, p->sys_nstep, q.st, q.aux())))
             return set_err(MGPU_ERR_CUDA, "large-N preparation", e);
         if ((phases & 2) && (e = run_big_prop(g, p->iprop, p->d_sys, y_dev, nodes_dev, status_dev, kfail_dev,
                                               q.st, q.aux())))
             return set_err(MGPU_ERR_CUDA, "large-N propagation", e);
-        if ((e = cudaEventRecord(q.done, q.st))) return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
     }
     // the small-N buckets beside them: the first with jobs on the caller's
     // stream, each of the others on one of its own
@@ -2121,12 +2121,13 @@ int mgpu_plan_run_device_phases(mgpu_plan *p, double *y_dev, int *nodes_dev, int
     for (size_t b = 0; b < p->bucket_ids.size(); ++b) {
         if (kBuckets[p->bucket_ids[b]].kind == KIND_BIG) continue;
         const bool jobs = p->job_count[b] > 0;
-        const int side = jobs && fork ? nth - 1 : -1;
+        const int side = jobs && own_streams ? nth - 1 : -1;
         nth += jobs;
         cudaStream_t bs = st;
         if (side >= 0) {
-            bs = p->sstreams[side].st;
-            if ((e = cudaStreamWaitEvent(bs, p->ev_in, 0))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
+            const mgpu_plan::SmallStream &q = p->sstreams[side];
+            bs = q.st;
+            if ((e = fork.to(q.st, q.done))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
         }
         for (int s0 = 0; prep && s0 < p->sys_count[b]; s0 += 65535)
             if ((e = launch_prep(p->bucket_ids[b], p->max_nstep[b], std::min(65535, p->sys_count[b] - s0), bs,
@@ -2136,15 +2137,9 @@ int mgpu_plan_run_device_phases(mgpu_plan *p, double *y_dev, int *nodes_dev, int
             (e = launch_prop(p->iprop, p->bucket_ids[b], p->job_count[b], p->smem[b], p->vl_smem[b], bs, p->d_sys,
                              p->d_jobs + p->job_begin[b], y_dev, nodes_dev, status_dev, kfail_dev)))
             return set_err(MGPU_ERR_CUDA, "launching the propagation kernel", e);
-        if (side >= 0 && (e = cudaEventRecord(p->sstreams[side].done, bs)))
-            return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     }
     // the caller's stream waits for every bucket
-    for (size_t i = 0; fork && i < p->sstreams.size(); ++i)
-        if ((e = cudaStreamWaitEvent(st, p->sstreams[i].done, 0))) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
-    for (size_t i = 0; i < p->big.size(); ++i)
-        if ((e = cudaStreamWaitEvent(st, p->bstreams[i].done, 0)))
-            return set_err(MGPU_ERR_CUDA, "ordering the large-N work", e);
+    if ((e = fork.join())) return set_err(MGPU_ERR_CUDA, "ordering the buckets", e);
     return MGPU_OK;
 }
 
