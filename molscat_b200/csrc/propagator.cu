@@ -47,9 +47,9 @@ struct SysDev {
     const double *rtab; // [2*nstep+1]
     const double *ptab; // [2*nstep+1][nham]
     double *q;          // LDMD: [nstep][T*T][ntiles] 2HQ(C_k)
-    double *wt;         // LDMD one-warp kernels or null: [nstep+1][ntiles][64] coupling sum
-                        // sum_l VL_l P_l(R) at R_0, R_2, .., R_2nstep (fragment layout)
-    double *wd;         // LDMD one-warp kernels or null: [nstep][npad] its diagonal at R_1, R_3, ..
+    double *wt;         // LDMD one-warp kernels or null (optional_table_doubles): [nstep+1][ntiles][64]
+                        // coupling sum sum_l VL_l P_l(R) at R_0, R_2, .., R_2nstep (fragment layout)
+    double *wd;         // beside wt: [nstep][npad] its diagonal at R_1, R_3, ..
     int *prep;          // LDMD: [0] negative pivots of all U inversions (NSAVE), [1] status, [2] kfail
     const volatile long long *ctl;  // plan's stop controls (device memory) or null: stop_requested
 };
@@ -974,6 +974,7 @@ static int set_err(int code, const char *what, cudaError_t e = cudaSuccess)
     else
         snprintf(buf, sizeof buf, "%s", what);
     g_last_error = buf;
+    if (e != cudaSuccess) cudaGetLastError();  // reported here: not to the next launch check
     return code;
 }
 
@@ -1236,6 +1237,27 @@ static cudaError_t big_invert(const big::MatDesc *md, int M, int nt, const big::
 
 static unsigned big_ew_blocks(size_t td) { return (unsigned)std::min<size_t>((td + big::EW_THREADS - 1) / big::EW_THREADS, 256); }
 
+// The coupling-sum tables (SysDev::wt and wd) of N 41-64, in doubles; 0 where a
+// system has none or cannot do without.  wt is as large as the 2HQ(C) table, so
+// a system that fits the device without them must not be refused for them: they
+// are placed after everything else and only in memory that is plentiful
+// (kTableShare), and the step kernel forms the sums itself where they are
+// missing, bit for bit the same: N = 60, 4000 jobs, 170 us a step with them, 253
+// (NHAM 6) and 426 (NHAM 24) without.
+static size_t optional_table_doubles(int iprop, int b, int nstep)
+{
+    if (iprop != MGPU_PROP_LDMD || kBuckets[b].kind != KIND_FRAG8 || kBuckets[b].nt <= 5) return 0;
+    return ((size_t)nstep + 1) * matrix_elems(b) + (size_t)nstep * bucket_npad(b);
+}
+// such tables take no more than this part of the memory that is free
+constexpr size_t kTableShare = 8;
+
+static void set_tables(SysDev &d, int b, double *t)
+{
+    d.wt = t;
+    d.wd = t ? t + ((size_t)d.nstep + 1) * matrix_elems(b) : nullptr;
+}
+
 // One system in bucket b's tile layout on the device: VL/IV tiled (sumlam.f
 // pair order), EINT/CENT padded, radial tables, MDPROP 2HQ(C) storage.
 static int build_sysdev(const mgpu_coupling &c, const mgpu_grid &g, int iprop, int b, SysDev &d, const AllocFn &al,
@@ -1295,7 +1317,7 @@ static int build_sysdev(const mgpu_coupling &c, const mgpu_grid &g, int iprop, i
     if (iprop == MGPU_PROP_LDMD && (e = alloc_n(al, &dq, (size_t)g.nstep * TT * nt)))
         return set_err(MGPU_ERR_NOMEM, "allocating the 2HQ(C) table", e);
     double *dwt = nullptr, *dwd = nullptr;
-    if (iprop == MGPU_PROP_LDMD && kBuckets[b].kind == KIND_FRAG8 &&
+    if (iprop == MGPU_PROP_LDMD && kBuckets[b].kind == KIND_FRAG8 && !optional_table_doubles(iprop, b, g.nstep) &&
         ((e = alloc_n(al, &dwt, ((size_t)g.nstep + 1) * TT * nt)) || (e = alloc_n(al, &dwd, (size_t)g.nstep * npad))))
         return set_err(MGPU_ERR_NOMEM, "allocating the coupling-sum tables", e);
     d.vlt = dv;
@@ -1807,6 +1829,35 @@ static int build_s(mgpu_plan *p)
     return MGPU_OK;
 }
 
+// The optional coupling-sum tables of a plan's systems, after everything else
+// it holds and beside what it may still allocate (Y, outputs, S matrices and
+// their scratch, the asymptotic-basis buffers).
+static void place_tables(mgpu_plan *p, std::vector<SysDev> &hs)
+{
+    size_t left = 0;
+    bool asked = false;
+    for (int s = 0; s < p->nsys; ++s) {
+        const size_t t = optional_table_doubles(p->iprop, p->sys_bucket[s], p->sys_nstep[s]) * sizeof(double);
+        if (t == 0 || p->sys_owner[s] != s) continue;
+        if (!asked) {
+            asked = true;
+            size_t free = 0, total = 0;
+            const size_t later = (3 * p->yelems + 2 * p->selems + p->sscr_elems) * sizeof(double) +
+                                 3 * (size_t)p->njobs * sizeof(int);
+            if (cudaMemGetInfo(&free, &total) == cudaSuccess && free > later) left = (free - later) / kTableShare;
+        }
+        double *d = nullptr;
+        if (t > left || p->dalloc(&d, t / sizeof(double)) != cudaSuccess) break;
+        left -= t;
+        set_tables(hs[s], p->sys_bucket[s], d);
+    }
+    cudaGetLastError();
+    for (int s = 0; s < p->nsys; ++s) {  // the systems that use another's tables
+        hs[s].wt = hs[p->sys_owner[s]].wt;
+        hs[s].wd = hs[p->sys_owner[s]].wd;
+    }
+}
+
 int mgpu_plan_create(mgpu_plan **out, int iprop, int nsys, const mgpu_coupling *systems,
                      const mgpu_grid *grids, int njobs, const int *job_sys, const double *job_ered)
 {
@@ -1918,10 +1969,6 @@ int mgpu_plan_create(mgpu_plan **out, int iprop, int nsys, const mgpu_coupling *
         }
     }
     for (int s = 0; s < nsys; ++s) hs[s].ctl = p->d_ctl;
-    if ((e = upload(p, &p->d_sys, hs.data(), hs.size()))) {
-        delete p;
-        return set_err(MGPU_ERR_NOMEM, "uploading system descriptors", e);
-    }
 
     // jobs: caller-order Y offsets; device order sorted by bucket then system
     p->yoff.resize(njobs);
@@ -2071,6 +2118,11 @@ int mgpu_plan_create(mgpu_plan **out, int iprop, int nsys, const mgpu_coupling *
     if (p->s_ok && (rc0 = build_s(p))) {
         delete p;
         return rc0;
+    }
+    place_tables(p, hs);
+    if ((e = upload(p, &p->d_sys, hs.data(), hs.size()))) {
+        delete p;
+        return set_err(MGPU_ERR_NOMEM, "uploading system descriptors", e);
     }
     *out = p;
     return MGPU_OK;

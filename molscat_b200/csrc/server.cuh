@@ -37,6 +37,9 @@ struct mgpu_server {
     std::vector<SysDev> hs;
     std::vector<int> sys_n, sys_nstep, sys_bucket, sys_nham;
     std::vector<void *> allocs;
+    std::vector<double *> tables;  // per system, or null: the optional coupling-sum tables
+    size_t table_bytes = 0;
+    bool launching = false;        // the scheduler is queueing a batch (without the mutex)
     cudaStream_t reg = nullptr, reg_side = nullptr;
     cudaEvent_t reg_evf = nullptr, reg_evj = nullptr;
     // requests
@@ -81,6 +84,9 @@ struct mgpu_server {
     void loop();
     bool retire();
     bool admit();
+    int register_system(const mgpu_coupling &c, const mgpu_grid &g, int b);
+    size_t spare() const;
+    void drop_tables(std::unique_lock<std::mutex> &lk);
     int launch(Slot &sl, const std::vector<long long> &tickets, const std::vector<const Req *> &rq, int b, size_t bytes);
     size_t job_bytes(int b, int n) const;
 };
@@ -284,10 +290,13 @@ bool mgpu_server::admit()
             }
             for (long long tk : take) pending.erase(std::find(pending.begin(), pending.end(), tk));
             in_use += bytes;  // reserved before launching
+            launching = true;
         }
         const int rc = launch(*free_slot, take, rq, b, bytes);
         {
             std::lock_guard<std::mutex> lk(mu);
+            launching = false;
+            cv_done.notify_all();
             const double t = now();
             for (long long tk : take) {
                 Req &r = reqs[tk];
@@ -318,6 +327,114 @@ bool mgpu_server::admit()
         any = true;
     }
     return any;
+}
+
+// Device memory beyond the batches' budget: what is free, or freed batch memory
+// that the pool keeps for the next batch.
+size_t mgpu_server::spare() const
+{
+    size_t free = 0, total = 0;
+    uint64_t pooled = 0;
+    cudaMemPool_t pool;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) free = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &pooled) != cudaSuccess)
+        pooled = 0;
+    cudaGetLastError();
+    const size_t have = free + (size_t)pooled;
+    return have > budget ? have - budget : 0;
+}
+
+// Gives the optional tables back.  Running batches read them: none is being
+// queued and all have ended first (the lock, held on return, keeps the
+// scheduler from queueing the next one; it is released while waiting).
+void mgpu_server::drop_tables(std::unique_lock<std::mutex> &lk)
+{
+    cv_done.wait(lk, [&] { return !launching; });
+    for (Slot &sl : slots) cudaStreamSynchronize(sl.st);
+    for (size_t k = 0; k < tables.size(); ++k) {
+        if (!tables[k]) continue;
+        set_tables(hs[k], sys_bucket[k], nullptr);
+        if (cudaMemcpyAsync(d_sys + k, &hs[k], sizeof(SysDev), cudaMemcpyHostToDevice, reg) != cudaSuccess ||
+            cudaStreamSynchronize(reg) != cudaSuccess)
+            continue;  // the descriptor still names it
+        cudaFree(tables[k]);
+        tables[k] = nullptr;
+        table_bytes -= optional_table_doubles(iprop, sys_bucket[k], sys_nstep[k]) * sizeof(double);
+    }
+}
+
+// System number nsys: its tables on the device, its descriptor in the registry
+// and, for MDPROP, its preparation.  Nothing of it is left after an error.
+int mgpu_server::register_system(const mgpu_coupling &c, const mgpu_grid &g, int b)
+{
+    const int sid = nsys;
+    const size_t kept = allocs.size();
+    const AllocFn al = [this](void **q, size_t nb) {
+        cudaError_t e2 = cudaMalloc(q, nb);
+        if (e2 == cudaSuccess) allocs.push_back(*q);
+        return e2;
+    };
+    const UploadFn up = [this](void *dst, const void *src, size_t nb) {
+        cudaError_t e2 = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, reg);
+        return e2 ? e2 : cudaStreamSynchronize(reg);
+    };
+    SysDev d;
+    cudaError_t e;
+    int rc = build_sysdev(c, g, iprop, b, d, al, up);
+    double *t = nullptr;
+    const size_t tb = optional_table_doubles(iprop, b, g.nstep) * sizeof(double);
+    if (!rc) {
+        if (tb > 0 && table_bytes + tb <= spare() / kTableShare) {
+            if (cudaMalloc((void **)&t, tb) != cudaSuccess) {
+                cudaGetLastError();
+                t = nullptr;
+            }
+            set_tables(d, b, t);
+        }
+        table_bytes += t ? tb : 0;
+        d.prep = d_prep + 3 * sid;
+        if ((e = up(d_sys + sid, &d, sizeof d))) rc = set_err(MGPU_ERR_CUDA, "registering a system", e);
+        hs.push_back(d);
+        sys_n.push_back(c.n);
+        sys_nstep.push_back(g.nstep);
+        sys_bucket.push_back(b);
+        sys_nham.push_back(c.nham);
+        tables.push_back(t);
+    }
+    if (!rc) prep_reset_kernel<<<1, 128, 0, reg>>>(d_prep + 3 * sid, 1);
+    // counters, and for MDPROP the energy-independent 2HQ(C) table, once
+    if (!rc && iprop == MGPU_PROP_LDMD) {
+        if (kBuckets[b].kind == KIND_BIG) {
+            std::vector<void *> tmp;
+            const AllocFn tal = [&tmp](void **q, size_t nb) {
+                cudaError_t e2 = cudaMalloc(q, nb);
+                if (e2 == cudaSuccess) tmp.push_back(*q);
+                return e2;
+            };
+            BigBucket gb;
+            rc = setup_big(gb, iprop, b, nullptr, nullptr, 0, 0, {sid}, hs, sys_n, sys_nstep, d_prep, tal, up);
+            if (!rc && (e = run_big_prep(gb, d_sys, sys_nstep, reg, BigAux{reg_side, reg_evf, reg_evj})))
+                rc = set_err(MGPU_ERR_CUDA, "large-N preparation", e);
+            cudaStreamSynchronize(reg);
+            for (void *q : tmp) cudaFree(q);
+        } else if ((e = launch_prep(b, g.nstep, 1, reg, d_sys, d_list + sid))) {
+            rc = set_err(MGPU_ERR_CUDA, "preparation", e);
+        }
+    }
+    if ((e = cudaStreamSynchronize(reg)) && !rc) rc = set_err(MGPU_ERR_CUDA, "registering a system", e);
+    if (rc) {
+        for (size_t k = kept; k < allocs.size(); ++k) cudaFree(allocs[k]);
+        allocs.resize(kept);
+        if (t) {
+            cudaFree(t);
+            table_bytes -= tb;
+        }
+        for (auto *v : {&sys_n, &sys_nstep, &sys_bucket, &sys_nham}) v->resize(std::min(v->size(), (size_t)sid));
+        hs.resize(std::min(hs.size(), (size_t)sid));
+        tables.resize(std::min(tables.size(), (size_t)sid));
+    }
+    return rc;
 }
 
 void mgpu_server::loop()
@@ -361,6 +478,8 @@ mgpu_server::~mgpu_server()
         if (sl.st) cudaStreamDestroy(sl.st);
     }
     if (reg) cudaStreamSynchronize(reg);
+    for (double *p : tables)
+        if (p) cudaFree(p);
     for (void *p : allocs) cudaFree(p);
     if (reg_evf) cudaEventDestroy(reg_evf);
     if (reg_evj) cudaEventDestroy(reg_evj);
@@ -390,6 +509,7 @@ int mgpu_server_create(mgpu_server **out, int iprop, size_t hbm_budget_bytes, in
     s->sys_nstep.reserve(max_systems);
     s->sys_bucket.reserve(max_systems);
     s->sys_nham.reserve(max_systems);
+    s->tables.reserve(max_systems);
     cudaError_t e;
     int lo = 0, hi = 0;
     if ((e = cudaGetDevice(&s->dev)) || (e = cudaDeviceGetStreamPriorityRange(&lo, &hi))) {
@@ -445,54 +565,17 @@ int mgpu_server_add_system(mgpu_server *s, const mgpu_coupling *c, const mgpu_gr
     int rc = check_coupling(c, g, s->iprop);
     if (rc) return rc;
     cudaSetDevice(s->dev);
-    std::lock_guard<std::mutex> lk(s->mu);
-    if (s->nsys >= s->cap) return set_err(MGPU_ERR_UNSUPPORTED, "server system capacity reached");
-    const int sid = s->nsys;
     const int b = bucket_for(c->n, s->iprop);
-    const AllocFn al = [s](void **q, size_t nb) {
-        cudaError_t e2 = cudaMalloc(q, nb);
-        if (e2 == cudaSuccess) s->allocs.push_back(*q);
-        return e2;
-    };
-    const UploadFn up = [s](void *dst, const void *src, size_t nb) {
-        cudaError_t e2 = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, s->reg);
-        return e2 ? e2 : cudaStreamSynchronize(s->reg);
-    };
-    SysDev d;
-    if ((rc = build_sysdev(*c, *g, s->iprop, b, d, al, up))) return rc;
-    d.prep = s->d_prep + 3 * sid;
-    cudaError_t e;
-    if ((e = up(s->d_sys + sid, &d, sizeof d))) return set_err(MGPU_ERR_CUDA, "registering a system", e);
-    s->hs.push_back(d);
-    s->sys_n.push_back(c->n);
-    s->sys_nstep.push_back(g->nstep);
-    s->sys_bucket.push_back(b);
-    s->sys_nham.push_back(c->nham);
-    // counters, and for MDPROP the energy-independent 2HQ(C) table, once
-    prep_reset_kernel<<<1, 128, 0, s->reg>>>(s->d_prep + 3 * sid, 1);
-    if (s->iprop == MGPU_PROP_LDMD) {
-        if (kBuckets[b].kind == KIND_BIG) {
-            std::vector<void *> tmp;
-            const AllocFn tal = [&tmp](void **q, size_t nb) {
-                cudaError_t e2 = cudaMalloc(q, nb);
-                if (e2 == cudaSuccess) tmp.push_back(*q);
-                return e2;
-            };
-            BigBucket gb;
-            rc = setup_big(gb, s->iprop, b, nullptr, nullptr, 0, 0, {sid}, s->hs, s->sys_n, s->sys_nstep, s->d_prep,
-                           tal, up);
-            if (!rc && (e = run_big_prep(gb, s->d_sys, s->sys_nstep, s->reg, BigAux{s->reg_side, s->reg_evf, s->reg_evj})))
-                rc = set_err(MGPU_ERR_CUDA, "large-N preparation", e);
-            cudaStreamSynchronize(s->reg);
-            for (void *q : tmp) cudaFree(q);
-            if (rc) return rc;
-        } else if ((e = launch_prep(b, g->nstep, 1, s->reg, s->d_sys, s->d_list + sid))) {
-            return set_err(MGPU_ERR_CUDA, "preparation", e);
-        }
+    std::unique_lock<std::mutex> lk(s->mu);
+    for (bool dropped = false;; dropped = true) {
+        if (s->nsys >= s->cap) return set_err(MGPU_ERR_UNSUPPORTED, "server system capacity reached");
+        rc = s->register_system(*c, *g, b);
+        if (rc != MGPU_ERR_NOMEM || s->table_bytes == 0 || dropped) break;
+        s->drop_tables(lk);  // another thread may register a system meanwhile
     }
-    if ((e = cudaStreamSynchronize(s->reg))) return set_err(MGPU_ERR_CUDA, "registering a system", e);
-    s->nsys = sid + 1;
-    *sys_id = sid;
+    if (rc) return rc;
+    *sys_id = s->nsys++;
+    if (s->table_bytes > 0 && s->spare() == 0) s->drop_tables(lk);  // the batches' budget comes first
     return MGPU_OK;
 }
 
