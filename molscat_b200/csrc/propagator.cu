@@ -639,8 +639,19 @@ __global__ void __launch_bounds__(256) pivot_reciprocal_probe_kernel(const doubl
 #ifndef MGPU_CTA_BUCKETS
 #define MGPU_CTA_BUCKETS(X) X(10, 4, 8) X(12, 8, 8) X(14, 8, 8) X(16, 8, 12) X(20, 12, 12) X(25, 16, 16)
 #endif
-// Few jobs: the shape for them fills no more than one wave of the 148 SMs.
-static bool few_jobs(int njobs, int warps_few) { return njobs <= 148 * (warps_few <= 8 ? 2 : 1); }
+// Few jobs: the shape for them, `ctas` of which an SM holds, fills no more than
+// one wave of the device's SMs.
+static bool few_jobs(int njobs, int ctas)
+{
+    static std::atomic<int> sms[64];  // by device, 0: not asked yet
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if ((n = sms[dev].load()) == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+        sms[dev].store(n);
+    }
+    return njobs <= n * ctas;
+}
 
 // NT of the large-N buckets (matrices in global memory, 64 pivots a round):
 // N up to 1024 in steps of 64
@@ -877,7 +888,8 @@ static cudaError_t launch_prop(int iprop, int b, int njobs, size_t smem, int vl_
         switch (nt) {
 #define X(t, w, wf)                                                                                  \
     case t:                                                                                          \
-        return few_jobs(njobs, wf) ? launch_cta<t, wf>(iprop, njobs, st, sys, jobs, y, nodes, status, kfail) \
+        static_assert(wf > 8 || 2 * cta::CSmem<t, wf>::bytes(true) <= 227 * 1024, "two CTAs an SM, as their registers allow"); \
+        return few_jobs(njobs, cta::min_ctas<wf>()) ? launch_cta<t, wf>(iprop, njobs, st, sys, jobs, y, nodes, status, kfail) \
                                    : launch_cta<t, w>(iprop, njobs, st, sys, jobs, y, nodes, status, kfail);
             MGPU_CTA_BUCKETS(X)
 #undef X
