@@ -47,9 +47,14 @@ struct CG {
     static constexpr int TW = W - 1;                                // tile warps
     // The factoring warp's chain of DFMAs waits for the DMMAs of the other warps on its
     // scheduler's FP64 pipe.  At NT = 14 and 20 those warps (3, 7, .. of 4n) take LN / LDEN of
-    // the others' tiles: LDMD, 1184 jobs, N = 106 6.87 -> 7.37 TFLOP/s, N = 150 6.91 -> 7.23
-    // (48 jobs 2.25 -> 2.34).  Elsewhere it costs a tile slot or gives nothing: N = 128
-    // 8.50 -> 8.29, N = 199 7.70 -> 7.40, N = 72 on four warps has no such warp.
+    // the others' tiles.  It costs registers (spill loads of the step kernels at NT = 14: LDMD
+    // 168 -> 624 bytes a thread, LDPROP 68 -> 812, LDMG 28 -> 376) and is the faster all the
+    // same, us a step without -> with: N = 106, 1184 jobs, LDMD 430 -> 401, LDMG 1221 -> 1143,
+    // LDPROP 703 -> 709 (no difference; 296 jobs 176 -> 171), 96 jobs LDMD 82.5 -> 81.8, LDMG 251
+    // -> 247; N = 150, 1184 jobs, LDMD 1189 -> 1138, LDMG 3299 -> 3189, 48 jobs LDMD 147 -> 141.
+    // Not so elsewhere: N = 90 (any number of jobs) no difference, N = 128, 1184 jobs, LDMD 610
+    // -> 623, LDMG 1555 -> 1562 (but LDPROP 1314 -> 1262), N = 199, 592 jobs, LDMD 1236 -> 1292.
+    // N = 72 in its shape of eight warps for few jobs would gain 2 %.
     static constexpr int LIGHT = NT == 14 || NT == 20 ? TW / 4 : 0;
     static constexpr int LN = W <= 8 ? 2 : 4, LDEN = W <= 8 ? 3 : 5;
     // tiles of one of the other warps when there are `ntiles` off the diagonal
@@ -62,8 +67,8 @@ struct CG {
     static constexpr int TD = NTL * 64;                             // doubles of one tiled matrix
     // pitch of the panel and operand columns in 16-byte pairs: 2 mod 8, so that the
     // eight lanes of an access phase meet eight bank groups; eight rows past the
-    // matrix, always zero, for the slots that hold no tile (and up to 32 rows read past
-    // the last tile row when the diagonal tiles are taken by fours)
+    // matrix, always zero, for the slots that hold no tile (and read past the last tile
+    // row where the diagonal tiles are taken by twos and their number is odd)
     static constexpr int LD = NPAD + 10;
 };
 
@@ -81,7 +86,7 @@ struct CSmem {
     static constexpr int PAN = 0;                       // panel [4][LD] pairs of columns
     static constexpr int XS = PAN + 8 * C::LD;          // X operands [4][LD] pairs (block 1, block 2)
     static constexpr int BS = XS + 8 * C::LD;           // B operands
-    static constexpr int DG = BS + 8 * C::LD;           // the diagonal tiles, to a whole four
+    static constexpr int DG = BS + 8 * C::LD;           // the diagonal tiles and room for one more (rounded up to four)
     static constexpr int FB = DG + 64 * ((NT + 3) / 4 * 4);             // Fact
     static constexpr int VEC = FB + Fact::SIZE;         // y14, y14', y23 by channel, twice (step parity)
     static constexpr int PARK = VEC + 6 * C::NPAD + 8;  // LDJ: the parked Z (eight doubles of slack for empty slots' reads)

@@ -7,8 +7,11 @@
 // one warp reads or writes a tile as 512 contiguous bytes.
 // VL is stored [term][t][l][s]; the 2HQ(C) table [step][t][l][s].
 //
-// Padding channels (N .. 8 NT - 1) are uncoupled; every kernel gives them a
-// positive diagonal before an inversion, so the sweep needs no test for them.
+// Padding channels (N .. 8 NT - 1) are uncoupled; every kernel gives those that
+// share a pivot block with a real channel a positive diagonal before an
+// inversion, so the sweep needs no test for them.  A half tile that is all
+// padding is not swept (warp_sweep_invert), so its diagonal is arbitrary:
+// LDPROP's drifts by -4.125 a step, LDMG's by 2/(a_k h) a stage.
 #pragma once
 #include "warp_dmma.cuh"
 

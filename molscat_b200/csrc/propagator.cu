@@ -627,9 +627,7 @@ __global__ void __launch_bounds__(256) pivot_reciprocal_probe_kernel(const doubl
 // bucket dispatch
 // ---------------------------------------------------------------------------
 #define MGPU_BUCKETS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(16)
-#ifndef MGPU_FRAG_BUCKETS
 #define MGPU_FRAG_BUCKETS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8)
-#endif
 // (NT, warps, warps in a launch of few jobs) of the one-CTA-per-matrix buckets,
 // N = 8*NT up to 200.  The results do not depend on the warps.  Measured, LDMD,
 // TFLOP/s with 1184 jobs: N = 72 6.3 on 4 warps (four CTAs an SM) against 4.5 on
@@ -665,22 +663,21 @@ enum { KIND_TILE4 = 0, KIND_FRAG8 = 1, KIND_CTA8 = 2, KIND_BIG = 3 };
 struct Bucket {
     int kind;
     int nt;
-    int warps;  // KIND_CTA8
 };
 
 // 8x8-fragment buckets first (one warp for N <= 64, one CTA up to 200), then
 // the 4x4 register tiles (N <= 64).
 static const Bucket kBuckets[] = {
-#define X(nt) {KIND_FRAG8, nt, 1},
+#define X(nt) {KIND_FRAG8, nt},
     MGPU_FRAG_BUCKETS(X)
 #undef X
-#define X(nt, w, wf) {KIND_CTA8, nt, w},
+#define X(nt, w, wf) {KIND_CTA8, nt},
     MGPU_CTA_BUCKETS(X)
 #undef X
-#define X(nt) {KIND_BIG, nt, 0},
+#define X(nt) {KIND_BIG, nt},
     MGPU_BIG_BUCKETS(X)
 #undef X
-#define X(nt) {KIND_TILE4, nt, 0},
+#define X(nt) {KIND_TILE4, nt},
     MGPU_BUCKETS(X)
 #undef X
 };
@@ -697,10 +694,14 @@ static int ntiles_of(int b) { return kBuckets[b].nt * (kBuckets[b].nt + 1) / 2; 
 static size_t tile_elems(int b) { return (size_t)bucket_edge(b) * bucket_edge(b); }  // doubles per tile
 static size_t matrix_elems(int b) { return tile_elems(b) * ntiles_of(b); }         // doubles per tiled matrix
 
-// LDJ keeps two tiled matrices in shared memory: CTA buckets up to N = 128.
 static bool is_ldmg(int iprop) { return iprop == MGPU_PROP_LDMG4 || iprop == MGPU_PROP_LDMG5; }
 
 // LDMG runs on the fragment-layout families: one warp, one CTA, batched large N.
+// LDPROP leaves the one-CTA kernels at N = 128: above, they are faster only with
+// 80 jobs or more (N = 199, TFLOP/s against the large-N kernels': 128 jobs 6.33
+// against 4.89, 48 jobs 2.40 against 3.73, 4 jobs 0.20 against 0.53), and the
+// number of jobs must not choose the family: a batch's results would differ from
+// those of its single calls.
 static bool bucket_allows(int b, int iprop)
 {
     if (is_ldmg(iprop)) return kBuckets[b].kind != KIND_TILE4;
@@ -1813,7 +1814,8 @@ static int build_s(mgpu_plan *p)
         }
     }
     p->selems = so;
-    // one CTA of the larger jobs' kernel fills an SM's threads, so it may take its shared memory too
+    // a CTA of the larger jobs' kernel may take all of an SM's shared memory (without the matrices two
+    // CTAs of 1024 threads would fit)
     p->s_moff_g = (p->s_smem_g + 15) / 16 * 2;
     const size_t room = smx::kSmemG / sizeof(double) - std::min(smx::kSmemG / sizeof(double), p->s_moff_g);
     for (size_t m : mats)

@@ -13,8 +13,9 @@
 //     A_ij  -= sum_k c_k(i) c_k(j) / delta_k        (i, j not in P)
 //     A_iP   = A_iP D^{-1} ,  A_PP = -D^{-1}
 // which after all blocks leaves -A^{-1}.  The trailing update is the scalar
-// sweep's own sum of rank-one terms, so the block sweep keeps its rounding
-// behaviour; forming D^{-1} first and updating with A_iP D^{-1} A_Pj instead
+// sweep's own rank-one terms (the one-warp sweep adds a block's four in the
+// order 3, 2, 1, 0, the others 0, 1, 2, 3), so the block sweep keeps its
+// rounding behaviour; forming D^{-1} first and updating with A_iP D^{-1} A_Pj instead
 // loses accuracy when a pivot is small next to its neighbours.  As in
 // tiles.cuh the entries of row/column block P are zeroed first and the operands
 // carry the pivot block, so every lower tile gets the same update
@@ -74,13 +75,9 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b,
 // triangle of d (the upper triangle is ignored), pivot by pivot as the scalar
 // sweep meets them.  On return d holds the block's operands:
 //     d[k][k] = 1/delta_k ,  d[i][k] = Lam[i][k] (i > k) ,  d[k][i] = 0
-// with Lam = L^{-1} (unit lower).  Negative pivots of the first `nreal` rows
-// are added to cnt; the rest are padding, zero off the diagonal, and taken as
-// exact unit pivots (not counted, never singular).
-__device__ __forceinline__ void ldl_block4(double d[4][4], int nreal, int &cnt, int &flags)
+// with Lam = L^{-1} (unit lower).  Negative pivots are added to cnt.
+__device__ __forceinline__ void ldl_block4(double d[4][4], int &cnt, int &flags)
 {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d[i][i] = (i >= nreal) ? 1.0 : d[i][i];
     double l[4][4], rd[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -111,16 +108,6 @@ __device__ __forceinline__ void ldl_block4(double d[4][4], int nreal, int &cnt, 
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) d[i][j] = (i == j) ? rd[i] : (i > j ? lam[i][j] : 0.0);
-}
-
-// This lane's share of the block operands (ldl_block4 layout in f): row q of
-// Lam below the diagonal (lq[m], m < q; zero for m >= q) and 1/delta_q.
-__device__ __forceinline__ void lane_operands(const double (&f)[4][4], int q, double (&lq)[3], double &rq)
-{
-    lq[0] = (q == 1) ? f[1][0] : (q == 2) ? f[2][0] : (q == 3) ? f[3][0] : 0.0;
-    lq[1] = (q == 2) ? f[2][1] : (q == 3) ? f[3][1] : 0.0;
-    lq[2] = (q == 3) ? f[3][2] : 0.0;
-    rq = (q == 1) ? f[1][1] : (q == 2) ? f[2][2] : (q == 3) ? f[3][3] : f[0][0];
 }
 
 // ---- the one-warp sweep -----------------------------------------------------
@@ -156,7 +143,7 @@ __device__ __noinline__ int ldl_block4_any(double *blk)
 #pragma unroll
         for (int j = 0; j < 4; ++j) d[i][j] = j <= i ? blk[4 * i + j] : 0.0;
     int cnt = 0, flags = 0;
-    ldl_block4(d, 4, cnt, flags);
+    ldl_block4(d, cnt, flags);
     __syncwarp();
     if ((threadIdx.x & 31) == 0) {
 #pragma unroll
@@ -254,7 +241,10 @@ __device__ __forceinline__ void factor_block(double v, double *blk, int lane, bo
 }
 
 // -A^{-1} in place; returns the negative-pivot count, `bad` as in tiles.cuh.
-// Padding rows and columns are uncoupled and have a positive diagonal.
+// Padding rows and columns are uncoupled and have a positive diagonal where a
+// pivot block holds one beside a real channel.  A last half tile that is all
+// padding is neither pivoted nor counted: its diagonal stays what it was,
+// whatever that is.
 // ws: G<NT>::WSM doubles of shared memory owned by this warp.
 //
 // The loop runs over the tile columns with the pivot tile always the first:
