@@ -254,7 +254,7 @@ __device__ __forceinline__ void factor_block(double v, double *blk, int lane, bo
 // after NT turns the matrix stands in its own order again.  Every register index
 // is fixed and the code is two rounds long, whatever NT: unrolled over the
 // rounds it filled the instruction caches (7843 instructions a propagation step
-// at NT = 5; this form issues about 3000), and with the pivot tile first there
+// at NT = 5, N 33-36; this form issues 5561), and with the pivot tile first there
 // is no row of tiles left of it, whose panel entries would need transposing.
 // The next block is factored as soon as its tile has its update, beside the
 // other DMMAs of the round.
