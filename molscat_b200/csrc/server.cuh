@@ -14,7 +14,10 @@
 //   bucket in arrival order, as many as the batch limit and the free part of
 //   the HBM budget allow.  Each batch runs on its own stream slot, so batches
 //   of different buckets (and later arrivals) overlap on the device; a batch
-//   never waits for the others.  Per-batch memory comes from the
+//   never waits for the others.  The last free slot is kept a moment for a
+//   bucket that has no batch running (kLastSlotHold): requests that come in one
+//   by one would otherwise fill every slot with batches of one, and an arrival
+//   of another size would wait for a whole run.  Per-batch memory comes from the
 //   stream-ordered allocator and returns to it when the batch completes.
 // * Results do not depend on the batch a request lands in: every kernel
 //   propagates each job independently.
@@ -60,6 +63,7 @@ struct mgpu_server {
         cudaStream_t st = nullptr, side = nullptr;
         cudaEvent_t evf = nullptr, evj = nullptr, done = nullptr;
         bool busy = false;
+        int bucket = -1;  // of the running batch
         std::vector<long long> tickets;
         std::vector<size_t> yoff;
         std::vector<void *> dev;
@@ -87,6 +91,7 @@ struct mgpu_server {
     int register_system(const mgpu_coupling &c, const mgpu_grid &g, int b);
     size_t spare() const;
     void drop_tables(std::unique_lock<std::mutex> &lk);
+    std::deque<long long>::iterator next_admissible();
     int launch(Slot &sl, const std::vector<long long> &tickets, const std::vector<const Req *> &rq, int b, size_t bytes);
     size_t job_bytes(int b, int n) const;
 };
@@ -247,6 +252,27 @@ bool mgpu_server::retire()
     return any;
 }
 
+// How long a request whose bucket already has a batch running leaves the last
+// free slot to others, from its submission on: well under the run of a batch of
+// some size, long enough for the rest of a burst of requests to come in (a
+// 512 x 512 Y0 takes 0.4-1 ms to submit) and share its batch.
+constexpr double kLastSlotHold = 5e-3;
+
+// The oldest pending request that may have a slot now (with the mutex held).
+std::deque<long long>::iterator mgpu_server::next_admissible()
+{
+    int idle = 0;
+    for (const Slot &sl : slots) idle += sl.busy ? 0 : 1;
+    const double t = now();
+    return std::find_if(pending.begin(), pending.end(), [&](long long tk) {
+        const Req &r = reqs[tk];
+        if (idle > 1 || t - r.t[0] >= kLastSlotHold) return true;
+        for (const Slot &sl : slots)
+            if (sl.busy && sl.bucket == sys_bucket[r.sys]) return false;
+        return true;
+    });
+}
+
 // Admit pending requests onto free slots (called without the mutex).
 bool mgpu_server::admit()
 {
@@ -265,9 +291,10 @@ bool mgpu_server::admit()
         size_t bytes = 0;
         {
             std::lock_guard<std::mutex> lk(mu);
-            if (pending.empty()) break;
-            b = sys_bucket[reqs[pending.front()].sys];
-            for (auto it = pending.begin(); it != pending.end() && (int)take.size() < max_batch; ++it) {
+            const auto first = next_admissible();
+            if (first == pending.end()) break;
+            b = sys_bucket[reqs[*first].sys];
+            for (auto it = first; it != pending.end() && (int)take.size() < max_batch; ++it) {
                 const Req &r = reqs[*it];
                 if (sys_bucket[r.sys] != b) continue;
                 const size_t jb = job_bytes(b, sys_n[r.sys]);
@@ -278,12 +305,12 @@ bool mgpu_server::admit()
             }
             if (take.empty()) {
                 if (in_use > 0) break;  // wait for memory to free up
-                // the oldest request alone exceeds the budget
-                Req &r = reqs[pending.front()];
+                // that request alone exceeds the budget
+                Req &r = reqs[*first];
                 r.rc = MGPU_ERR_NOMEM;
                 r.state = 2;
                 r.t[2] = now();
-                pending.pop_front();
+                pending.erase(first);
                 cv_done.notify_all();
                 any = true;
                 continue;
@@ -323,6 +350,7 @@ bool mgpu_server::admit()
             cv_done.notify_all();
         } else {
             free_slot->busy = true;
+            free_slot->bucket = b;
         }
         any = true;
     }
