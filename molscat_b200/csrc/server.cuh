@@ -14,10 +14,11 @@
 //   bucket in arrival order, as many as the batch limit and the free part of
 //   the HBM budget allow.  Each batch runs on its own stream slot, so batches
 //   of different buckets (and later arrivals) overlap on the device; a batch
-//   never waits for the others.  The last free slot is kept a moment for a
-//   bucket that has no batch running (kLastSlotHold): requests that come in one
-//   by one would otherwise fill every slot with batches of one, and an arrival
-//   of another size would wait for a whole run.  Per-batch memory comes from the
+//   never waits for the others.  A large-N bucket with a batch running leaves
+//   the last free slot a moment to a registered bucket that has none
+//   (kLastSlotHold): large requests that come in one by one would otherwise fill
+//   every slot with batches of one, and an arrival of another size would wait for
+//   a whole run.  Per-batch memory comes from the
 //   stream-ordered allocator and returns to it when the batch completes.
 // * Results do not depend on the batch a request lands in: every kernel
 //   propagates each job independently.
@@ -39,6 +40,7 @@ struct mgpu_server {
     int *d_list = nullptr;  // d_list[s] = s
     std::vector<SysDev> hs;
     std::vector<int> sys_n, sys_nstep, sys_bucket, sys_nham;
+    std::vector<int> buckets;  // those with a system, each once
     std::vector<void *> allocs;
     std::vector<double *> tables;  // per system, or null: the optional coupling-sum tables
     size_t table_bytes = 0;
@@ -252,24 +254,29 @@ bool mgpu_server::retire()
     return any;
 }
 
-// How long a request whose bucket already has a batch running leaves the last
-// free slot to others, from its submission on: well under the run of a batch of
-// some size, long enough for the rest of a burst of requests to come in (a
-// 512 x 512 Y0 takes 0.4-1 ms to submit) and share its batch.
-constexpr double kLastSlotHold = 5e-3;
+// How long a large-N request whose bucket already has a batch running leaves the
+// last free slot to others, from its submission on: well under such a batch's
+// run (0.35 ms a step at N = 512), long enough for the rest of a burst of
+// requests to come in (a 512 x 512 Y0 takes 0.4-1 ms to submit) and share its
+// batch, which then takes hardly longer.  Not the one-warp and one-CTA buckets:
+// there a batch of one leaves most of the GPU free and a slot kept is time lost
+// (39 mixes of 16-96 requests, N 8-128: 3 % more time, up to 30 %).
+constexpr double kLastSlotHold = 3e-3;
 
 // The oldest pending request that may have a slot now (with the mutex held).
 std::deque<long long>::iterator mgpu_server::next_admissible()
 {
     int idle = 0;
     for (const Slot &sl : slots) idle += sl.busy ? 0 : 1;
+    auto runs = [&](int b) {
+        return std::any_of(slots.begin(), slots.end(), [b](const Slot &sl) { return sl.busy && sl.bucket == b; });
+    };
+    if (idle > 1 || std::all_of(buckets.begin(), buckets.end(), runs)) return pending.begin();
     const double t = now();
     return std::find_if(pending.begin(), pending.end(), [&](long long tk) {
         const Req &r = reqs[tk];
-        if (idle > 1 || t - r.t[0] >= kLastSlotHold) return true;
-        for (const Slot &sl : slots)
-            if (sl.busy && sl.bucket == sys_bucket[r.sys]) return false;
-        return true;
+        const int b = sys_bucket[r.sys];
+        return kBuckets[b].kind != KIND_BIG || t - r.t[0] >= kLastSlotHold || !runs(b);
     });
 }
 
@@ -603,6 +610,7 @@ int mgpu_server_add_system(mgpu_server *s, const mgpu_coupling *c, const mgpu_gr
     }
     if (rc) return rc;
     *sys_id = s->nsys++;
+    if (std::find(s->buckets.begin(), s->buckets.end(), b) == s->buckets.end()) s->buckets.push_back(b);
     if (s->table_bytes > 0 && s->spare() == 0) s->drop_tables(lk);  // the batches' budget comes first
     return MGPU_OK;
 }
