@@ -29,7 +29,10 @@ private:
     {
         cudaError_t e = cudaEventRecord(done, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(caller_, done, 0);
-        if (e != cudaSuccess) cudaStreamSynchronize(st);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(st);
+            cudaGetLastError();  // returned here, or behind an error reported already: not to the next launch check
+        }
         return e;
     }
 
